@@ -178,7 +178,7 @@ Layout layout(const PgeGrid &g)
     L.w_mom = take(8 * ws);
     L.w_count = take(8 * L.max_wave);
     L.w_death = take(L.max_wave);
-    L.w_desc = take(16 * ws);
+    L.w_rec = take(32 * ws);
     L.w_keys0 = take(8 * ws);
     L.w_keys1 = take(8 * ws);
     L.w_vals0 = take(4 * ws);
@@ -191,11 +191,9 @@ Layout layout(const PgeGrid &g)
     L.w_temp = take(L.w_temp_bytes);
     L.w_dth = take(4 * L.max_wave);
     L.w_keep = take(8 * L.max_wave);
-    L.w_act = take(8 * ws);
     L.w_park_n = take(4 * L.max_wave);
     L.w_park_k = take(4 * LAKE_PARKS * L.max_wave);
     L.w_park_rest = take(8 * LAKE_PARKS * L.max_wave);
-    L.w_fin = take(8 * ws);
     L.w_offsets = take(8 * (L.max_wave + 1));
     L.hand = take(16 * L.ncell);
     L.terr = take(16 * L.ncell);
@@ -325,7 +323,7 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
             oa.mom = a.rec_mom;
             oa.count = a.rec_count;
             oa.cap = (int)lay.cap;
-            oa.desc = ws_ptr<EntryDesc>(ws, lay.w_desc);
+            oa.rec = ws_ptr<EntryRec>(ws, lay.w_rec);
             oa.terr = ws_ptr<CellTerr>(ws, lay.terr);
             oa.L = a.L;
             oa.sediment = s->sediment;
@@ -340,7 +338,6 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
             oa.hand = ws_ptr<double2>(ws, lay.hand);
             oa.dth = ws_ptr<int32_t>(ws, lay.w_dth);
             oa.keep = ws_ptr<double>(ws, lay.w_keep);
-            oa.act = ws_ptr<double>(ws, lay.w_act);
             oa.p = *p;
             oa.stats = stats;
             oa.error = ws_ptr<int>(ws, lay.error);
@@ -384,10 +381,7 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
             ow.segscan = ws_ptr<int32_t>(ws, lay.w_segscan);
             ow.temp = ws_ptr<void>(ws, lay.w_temp);
             ow.temp_bytes = lay.w_temp_bytes;
-            ow.fin_kp = ws_ptr<double>(ws, lay.w_fin);
             ow.offsets = lay.cap >= COMPACT_CAP ? ws_ptr<long long>(ws, lay.w_offsets) : nullptr;
-            oa.lanes = p->apply_lanes > 0 ? p->apply_lanes : 1;
-            ow.max_blocks = (long long)sm_count() * ordered_blocks_per_sm(oa.lanes);
             const long long rec_warps =
                 (long long)sm_count() * (lateral ? droplet_blocks_per_sm_f64_lateral(32, false, s->route != nullptr)
                                          : s->route ? droplet_blocks_per_sm_f64_route(32, false)

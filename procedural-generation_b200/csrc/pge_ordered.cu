@@ -26,10 +26,14 @@
 //     death cell as the droplet's own last write there left it, so it is
 //     taken at that write and the death cell is handed on like any other;
 //   * a droplet's path through the wave is mostly its own entries one after
-//     another, so each entry's packed 16-byte descriptor, its cell's packed
-//     16-byte terrain and the cell's hand-off word are copied into a ring in
-//     shared memory several entries ahead (asynchronous copies, waited for
-//     by group count);
+//     another (on a wave's critical path 9 in 10 steps go from an entry to
+//     its droplet's next one, 1 in 10 over a hand-off of ~350 ns), so what
+//     one entry costs bounds the wave.  The rank kernel, which has every
+//     entry in parallel, therefore writes all that an entry reads -- its
+//     cell's terrain, whom to wait for, which neighbours in the list share
+//     or read its cell -- into one 32-byte record in list order, and the
+//     apply is left with two shared-memory reads, the arithmetic and the
+//     hand-off store;
 //   * the order-dependent float64 sums that nothing in the wave reads back
 //     -- the discharge and momentum tracks and the stockpile -- are summed
 //     after the apply, per cell, walking the sorted entries: (droplet,
@@ -53,7 +57,7 @@ inline int grid_for(long long n, int threads = 256)
     return (int)(b < 1 ? 1 : (b > 1048576 ? 1048576 : b));
 }
 
-constexpr long long kSpinLimit = 1LL << 22;  // ~ seconds of polling: far beyond any real hand-off
+constexpr int kSpinLimit = 1 << 24;  // ~ seconds of polling: far beyond any real hand-off
 // a waiting warp sleeps PGE_POLL_SLEEP_NS after every PGE_POLL_EVERY polls (a power of two)
 #ifndef PGE_POLL_EVERY
 #define PGE_POLL_EVERY 256
@@ -89,37 +93,11 @@ __device__ __forceinline__ void hand_load(const double2 *p, unsigned long long &
     asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(p) : "memory");
 }
 
-// the same read issued ahead of its use: no compiler barrier, the thread waits only where it uses the word
-__device__ __forceinline__ void hand_load_ahead(const double2 *p, unsigned long long &w0, unsigned long long &w1)
-{
-    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w0), "=l"(w1) : "l"(p));
-}
-
 __device__ __forceinline__ void hand_store(double2 *p, double acc, uint32_t count)
 {
     unsigned long long w0, w1;
     hand_pack(acc, count, w0, w1);
     asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" : : "l"(p), "l"(w0), "l"(w1));
-}
-
-// wait until the D earlier droplets of this wave that visit cell c have handed it on; acc = its net change
-__device__ __forceinline__ bool acquire(const double2 *hand, long long c, uint32_t epoch, int D, int *error, double &acc)
-{
-    const uint32_t want = epoch + (uint32_t)D;
-    unsigned long long w0, w1;
-    for (long long i = 0; i < kSpinLimit; i++) {
-        hand_load(hand + c, w0, w1);
-        if (D == 0 || hand_ready(w0, w1, want)) {  // D == 0: the wave's first visitor, no earlier writer
-            acc = hand_acc(w0, w1);
-            return true;
-        }
-        if ((i & (PGE_POLL_EVERY - 1)) == PGE_POLL_EVERY - 1) {
-            if (*(volatile int *)error) return false;  // another wait gave up: stop waiting
-            __nanosleep(PGE_POLL_SLEEP_NS);
-        }
-    }
-    atomicExch(error, 1);
-    return false;
 }
 
 // a cell this droplet holds and has written before: its own last write (coherent for the same thread)
@@ -151,7 +129,6 @@ __device__ __forceinline__ void cp_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-enum { OS_CLAMPED, OS_TOPEND, OS_DEFICIT, OS_LOSTOFF, OS_ERODED, OS_DEPOSITED, OS_N };
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -209,24 +186,46 @@ __global__ void ordered_flags_kernel(long long nslots, const unsigned long long 
     }
 }
 
+// whether an entry reads the next one's cell live: an erosion (its floor) and a final deposit (its ceiling) do, a step
+// deposit and a lake park do not
+__device__ __forceinline__ bool reads_next(double delta, float vol) { return vol != -3.0f && (delta < 0.0 || vol < 0.0f); }
+
 __global__ void ordered_rank_kernel(long long nslots, const unsigned long long *keys, const int32_t *vals, int cap,
                                     unsigned long long invalid, const int32_t *runscan, const int32_t *segscan,
-                                    const double *delta, const float *vol, EntryDesc *desc)
+                                    const double *delta, const float *vol, const int64_t *count,
+                                    const CellTerr *terr, uint32_t epoch, EntryRec *rec)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nslots; i += (long long)gridDim.x * blockDim.x) {
         const unsigned long long k = keys[i];
         if (k == invalid) continue;
-        const int32_t s = vals[i];
-        const uint32_t D = (uint32_t)(runscan[i] - runscan[segscan[i]]);
-        bool lst = true;
-        if (i + 1 < nslots) lst = keys[i + 1] != k || vals[i + 1] / cap != s / cap;
-        const bool fst = i == 0 || keys[i - 1] != k || vals[i - 1] / cap != s / cap;
-        EntryDesc d;
-        d.cell = (int32_t)k;
-        d.dflags = D | (lst ? ENTRY_LAST : 0u) | (fst ? ENTRY_FIRST : 0u) | (vol[s] >= 0.0f ? ENTRY_STEP : 0u) |
-                   (vol[s] == -3.0f ? ENTRY_PARK : 0u);
-        d.delta = delta[s];
-        desc[s] = d;
+        const int32_t s = vals[i], q = s / cap, e = s - q * cap;
+        const CellTerr t = terr[k];
+        const float v = vol[s];
+        const double d = delta[s];
+        EntryRec r;
+        r.delta = d;
+        r.hs = t.hs;
+        r.base = t.base;
+        r.cell = (int32_t)k;
+        // the droplet's visits before and after this one are its neighbours in the sorted order
+        const int32_t back = i > 0 && keys[i - 1] == k && vals[i - 1] / cap == q ? s - vals[i - 1] : 0;
+        const int32_t fwd = i + 1 < nslots && keys[i + 1] == k && vals[i + 1] / cap == q ? vals[i + 1] - s : 0;
+        const uint32_t D = (uint32_t)(runscan[i] - runscan[segscan[i]]);  // distinct earlier droplets at the cell
+        const bool reads = e + 1 < count[q] && reads_next(d, v);
+        uint32_t f = (uint32_t)(back < APPLY_HIST ? back : APPLY_HIST);
+        if (fwd == 0) f |= ENTRY_LAST;
+        if (back == 0) f |= ENTRY_FIRST;
+        if (back != 0 || D == 0) f |= ENTRY_OPEN;
+        if (v >= 0.0f) f |= ENTRY_STEP;
+        if (t.active && v != -3.0f) f |= d < 0.0 ? ENTRY_ERO : ENTRY_DEP;
+        if (reads) f |= ENTRY_READS;
+        if (reads && fwd != 1) f |= ENTRY_NEEDS;
+        if (fwd == 1) f |= ENTRY_SAME;
+        if (e > 0 && (back == 1 || reads_next(delta[s - 1], vol[s - 1]))) f |= ENTRY_HELD;
+        if (fwd >= APPLY_HIST) f |= ENTRY_FAR;
+        r.flags = f;
+        r.turn = epoch + D;
+        rec[s] = r;
     }
 }
 
@@ -334,197 +333,102 @@ cudaError_t park_wave(const ParkWave &pw, cudaStream_t st)
 // the ordered apply
 // ---------------------------------------------------------------------------
 namespace {
-// prefetch depth: at entry k the copies of the last LOOKAHEAD entries may still be in flight; the cell data of
-// entry k + CELL_AHEAD and the descriptor of entry k + DESC_AHEAD are issued (the descriptor lands before its
-// cell data is issued, the cell data before its entry and the one before it are applied)
-#ifndef PGE_APPLY_LOOKAHEAD
-#define PGE_APPLY_LOOKAHEAD 1
+constexpr unsigned FULL = 0xffffffffu;
+// records of a droplet's list on chip: the chunk being applied, the next two and the one before (a power of two)
+constexpr int REC_RING = 128;
+// a waiting warp whose turn is n droplets away sleeps n * BACK_NS (at most BACK_MAX of them) between its looks
+#ifndef PGE_BACK_NS
+#define PGE_BACK_NS 64
 #endif
-constexpr int LOOKAHEAD = PGE_APPLY_LOOKAHEAD;
-constexpr int CELL_AHEAD = LOOKAHEAD + 2;
-constexpr int DESC_AHEAD = CELL_AHEAD + LOOKAHEAD + 1;
-constexpr int RING = DESC_AHEAD < 8 ? 8 : (DESC_AHEAD < 16 ? 16 : 32);  // entry slots per droplet (a power of two)
-static_assert(RING > DESC_AHEAD, "the ring holds every entry in flight");
-// two droplets per block: a block's warp slots free up as soon as its two droplets are done, so
-// concurrent passes (other worlds' waves on other streams) pack around the long-lived droplets
-constexpr int APPLY_THREADS = 64;
-// resident blocks asked of the register allocator: 8 gives the plain variant 70 registers without spills (its
-// own choice, 48 registers and 12 spilled bytes, was 2.5 % slower)
-#ifndef PGE_APPLY_MINB
-#define PGE_APPLY_MINB 8
+#ifndef PGE_BACK_MAX
+#define PGE_BACK_MAX 16
 #endif
 
-// one entry of a droplet's list as the apply reads it, filled by asynchronous copies
-struct alignas(16) Slot {
-    EntryDesc d;                // descriptor
-    unsigned long long spare[2];  // (the hand-off word is read into registers instead)
-    CellTerr t;                 // the cell's read-only terrain
-    double cap;                 // the slope erode cap (when on)
-    float2 route;               // the cell's packed routing surface and flag (with lakes)
+template <int N>
+struct Int {
+    static constexpr int value = N;
 };
-static_assert(sizeof(Slot) == 64, "slot layout");
-
-__device__ __forceinline__ void stage_desc(const OrderedArgs &a, Slot &s, long long e) { cp_cg16(&s.d, a.desc + e); }
-
-template <bool ECAP, bool LAKE>
-__device__ __forceinline__ void stage_cell(const OrderedArgs &a, Slot &s)
-{
-    const long long c = s.d.cell;
-    cp_cg16(&s.t, a.terr + c);
-    if (ECAP) cp_ca8(&s.cap, a.ecap + c);
-    if (LAKE) cp_ca8(&s.route, a.R + c);
-}
-
-// one entry's slot as registers: read one entry before it is applied, while the entry before it
-// computes, so that the apply's chain from entry to entry holds only its arithmetic
-struct Ent {
-    int32_t c;
-    uint32_t df;
-    double dlt, hs, cap;
-    float base;
-    uint32_t active;
-    unsigned long long h0, h1;
-    float2 route;
-};
-
-template <bool ECAP, bool LAKE>
-__device__ __forceinline__ Ent load_ent(const Slot &s)
-{
-    Ent e;
-    e.c = s.d.cell;
-    e.df = s.d.dflags;
-    e.dlt = s.d.delta;
-    e.hs = s.t.hs;
-    e.base = s.t.base;
-    e.active = s.t.active;
-    e.h0 = e.h1 = 0ull;  // read separately, one entry ahead
-    e.cap = ECAP ? s.cap : 0.0;
-    e.route = LAKE ? s.route : make_float2(0.f, 0.f);
-    return e;
-}
 
 // per droplet state carried from entry to entry
 struct Walk {
-    double deficit, surplus, prev_live, acc_c;
+    double deficit, surplus, prev_live;
     int clamped;
     int32_t death;
-    // this droplet's last three writes (cell, net change after it)
-    int32_t w1c, w2c, w3c;
-    double w1v, w2v, w3v;
-    bool sub_death, has_prev, have_c, ok;
+    bool sub_death;
 };
 
-// the net change of a cell this droplet is about to read: a recent write of its own, its own
-// earlier write (a revisit), the prefetched word once the D earlier droplets have handed the cell
-// on, or a wait for them
-__device__ __forceinline__ bool cell_value(const OrderedArgs &a, const Walk &w, int32_t c, uint32_t df,
-                                           unsigned long long h0, unsigned long long h1, double &acc)
-{
-    if (c == w.w1c) {
-        acc = w.w1v;
-        return true;
-    }
-    if (c == w.w2c) {
-        acc = w.w2v;
-        return true;
-    }
-    if (c == w.w3c) {
-        acc = w.w3v;
-        return true;
-    }
-    if (!(df & ENTRY_FIRST)) {
-        acc = own_value(a.hand, c);
-        return true;
-    }
-    const uint32_t D = df & ENTRY_D_MASK;
-    if (D == 0 || hand_ready(h0, h1, a.epoch + D)) {
-        acc = hand_acc(h0, h1);
-        return true;
-    }
-    return acquire(a.hand, c, a.epoch, (int)D, a.error, acc);
-}
 }  // namespace
 
 // One change-list entry against the live terrain (particle.py:934-1002): the erosion floor (the
 // base level or the cell itself, the next path cell's live surface nlive), the deposit ceilings (the
 // previous step's live surface, or for a final deposit the next, older path cell), the deficit and
-// surplus carried along the droplet's list.  acc is the cell's live net change; writes the new one
-// and the amount actually moved.
+// surplus carried along the droplet's list.  acc is the cell's live net change; returns the new one
+// and the amount actually moved (negative: eroded).
 template <bool ECAP, bool LAKE>
-__device__ __forceinline__ void entry_arith(const PgeParams &p, Walk &w, int32_t c, double dlt, bool is_step, bool act, double hs,
-                                            double b_c, double acc, bool has_next, double nlive, double capv, float2 route,
-                                            double &acc_new, double &amount)
+__device__ __forceinline__ double entry_arith(const PgeParams &p, Walk &w, const EntryRec &r, double acc, double nlive, double capv,
+                                              float2 route, double &amount)
 {
-    if (act) {
-        const double s_c = hs + acc;
-        if (dlt < 0.0) {
-            const double ew = -dlt;
-            double e_act = ew;
-            double room = p.iter_erode + acc;
-            if (ECAP) {
-                const double r2 = capv + acc;
-                if (r2 < room) room = r2;
-            }
-            if (e_act > room) e_act = room;
-            double floor_ = s_c >= b_c ? b_c : s_c;
-            // a lake bed is never eroded below its water level (particle.py:952-956)
-            if (LAKE && route.y >= 1.5f && (double)route.x > floor_) floor_ = (double)route.x;
-            if (has_next && nlive > floor_) floor_ = nlive;
-            if (e_act > s_c - floor_) e_act = s_c - floor_;
-            if (e_act < 0.0) e_act = 0.0;
-            if (e_act < ew) {
-                w.clamped++;
-                w.deficit += ew - e_act;
-            }
-            acc_new = acc - e_act;
-            amount = e_act;
-        } else {
-            double want = dlt + w.surplus;
-            w.surplus = 0.0;
-            if (w.deficit > 0.0) {
-                const double t = want < w.deficit ? want : w.deficit;
-                want -= t;
-                w.deficit -= t;
-            }
-            double d_act = want;
-            const double room = p.iter_deposit - acc;
-            if (d_act > room) d_act = room;
-            bool has_ref = false;
-            double ref_live = 0.0;
-            if (is_step) {
-                has_ref = w.has_prev;
-                ref_live = w.prev_live;
-            } else if (has_next) {
-                has_ref = true;
-                ref_live = nlive;
-            }
-            if (has_ref) {
-                double ceil_ = ref_live + p.dep_floor;
-                if (s_c < b_c && is_step) ceil_ -= p.dep_floor + p.fan_slope;
-                const double lim = ceil_ - s_c;
-                if (d_act > lim) d_act = lim;
-            }
-            if (s_c < b_c) {
-                const double lim = b_c - p.dep_floor - s_c;
-                if (d_act > lim) d_act = lim;
-            }
-            if (d_act < 0.0) d_act = 0.0;
-            if (d_act < want) w.clamped++;
-            w.surplus = want - d_act;
-            acc_new = acc + d_act;
-            amount = d_act;
-            if (!is_step && w.death < 0) w.death = c;
+    const uint32_t f = r.flags;
+    const double s_c = r.hs + acc, b_c = (double)r.base;
+    double acc_new = acc;
+    amount = 0.0;
+    if (f & ENTRY_ERO) {
+        const double ew = -r.delta;
+        double room = p.iter_erode + acc;
+        if (ECAP) {
+            const double r2 = capv + acc;
+            room = r2 < room ? r2 : room;
         }
-        if (c == w.death) w.sub_death = hs + acc_new < b_c;
-        if (is_step) {
-            w.has_prev = true;
-            w.prev_live = hs + acc_new;
+        double e_act = ew > room ? room : ew;
+        double floor_ = s_c >= b_c ? b_c : s_c;
+        // a lake bed is never eroded below its water level (particle.py:952-956)
+        if (LAKE) floor_ = route.y >= 1.5f && (double)route.x > floor_ ? (double)route.x : floor_;
+        floor_ = (f & ENTRY_READS) && nlive > floor_ ? nlive : floor_;
+        const double lim = s_c - floor_;
+        e_act = e_act > lim ? lim : e_act;
+        e_act = e_act < 0.0 ? 0.0 : e_act;
+        acc_new = acc - e_act;
+        amount = -e_act;
+        const bool less = e_act < ew;
+        w.clamped += less;
+        const double deficit = w.deficit + (ew - e_act);
+        w.deficit = less ? deficit : w.deficit;
+        const double live = r.hs + acc_new;
+        w.prev_live = (f & ENTRY_STEP) ? live : w.prev_live;  // (a bank cut is no step)
+    } else if (f & ENTRY_DEP) {
+        const bool below = s_c < b_c, is_step = (f & ENTRY_STEP) != 0;
+        const double got = r.delta + w.surplus;
+        double t = got < w.deficit ? got : w.deficit;
+        t = w.deficit > 0.0 ? t : 0.0;
+        const double want = got - t;
+        w.deficit -= t;
+        const double room = p.iter_deposit - acc;
+        double d_act = want > room ? room : want;
+        // the ceiling: the last step's live surface (none yet: infinite), for a final deposit the next, older path cell's
+        double ceil_ = (is_step ? w.prev_live : nlive) + p.dep_floor;
+        const double ceil_b = ceil_ - (p.dep_floor + p.fan_slope);
+        ceil_ = below && is_step ? ceil_b : ceil_;
+        const double lim1 = ceil_ - s_c;
+        d_act = (f & (ENTRY_STEP | ENTRY_READS)) && d_act > lim1 ? lim1 : d_act;
+        const double lim2 = b_c - p.dep_floor - s_c;
+        d_act = below && d_act > lim2 ? lim2 : d_act;
+        d_act = d_act < 0.0 ? 0.0 : d_act;
+        acc_new = acc + d_act;
+        amount = d_act;
+        w.clamped += d_act < want;
+        w.surplus = want - d_act;
+        const double live = r.hs + acc_new;
+        w.prev_live = is_step ? live : w.prev_live;
+        if (!is_step) {  // the final deposits end the list: the first one's cell takes the stockpile
+            w.death = w.death < 0 ? r.cell : w.death;
+            w.sub_death = r.cell == w.death ? live < b_c : w.sub_death;
         }
     }
+    return acc_new;
 }
 
 // a droplet's stockpile (particle.py:1019-1041) and its statistics, once its list is applied
-__device__ __forceinline__ void droplet_end(const OrderedArgs &a, const Walk &w, long long q, unsigned long long *sstat)
+__device__ __forceinline__ void droplet_end(const OrderedArgs &a, const Walk &w, long long q, long long eroded, long long deposited)
 {
     const PgeParams &p = a.p;
     long long topend = 0, lostoff = 0;
@@ -552,143 +456,184 @@ __device__ __forceinline__ void droplet_end(const OrderedArgs &a, const Walk &w,
     }
     a.dth[q] = dth;
     a.keep[q] = add;
-    if (w.clamped) atomicAdd(&sstat[OS_CLAMPED], (unsigned long long)w.clamped);
-    if (topend) atomicAdd(&sstat[OS_TOPEND], (unsigned long long)topend);
-    if (w.deficit > 0.0) atomicAdd(&sstat[OS_DEFICIT], (unsigned long long)fx_mass(w.deficit));
-    if (lostoff) atomicAdd(&sstat[OS_LOSTOFF], (unsigned long long)lostoff);
+    PgeStats *st = a.stats;
+    auto total = [](int64_t *dst, long long v) {
+        if (v) red_add(reinterpret_cast<long long *>(dst), v);
+    };
+    total(&st->clamped, w.clamped);
+    total(&st->to_pending_fx, topend);
+    if (w.deficit > 0.0) total(&st->deficit_out_fx, fx_mass(w.deficit));
+    total(&st->lost_offshore_fx, lostoff);
+    total(&st->eroded_fx, eroded);
+    total(&st->deposited_fx, deposited);
 }
 
-// the block's statistics to the pass totals (after a __syncthreads)
-__device__ __forceinline__ void flush_stats(const OrderedArgs &a, const unsigned long long *sstat)
-{
-    if (threadIdx.x < OS_N && sstat[threadIdx.x]) {
-        PgeStats *st = a.stats;
-        int64_t *dst = threadIdx.x == OS_CLAMPED ? &st->clamped
-                     : threadIdx.x == OS_TOPEND ? &st->to_pending_fx
-                     : threadIdx.x == OS_DEFICIT ? &st->deficit_out_fx
-                     : threadIdx.x == OS_LOSTOFF ? &st->lost_offshore_fx
-                     : threadIdx.x == OS_ERODED ? &st->eroded_fx
-                                                : &st->deposited_fx;
-        red_add(reinterpret_cast<long long *>(dst), (long long)sstat[threadIdx.x]);
-    }
-}
-
+// One warp a droplet: every lane runs the droplet's entries (the same values in all lanes), the lanes share the
+// copies of its records and the statistics of 32 entries at a time.
+//
+// Bound by the instructions of one entry on one warp (~110, 215-235 ns; 2048 droplets at work at once: 405), not
+// by memory.  What each choice measured, ns an entry without a wait: hand-off words read into registers ahead of
+// their use 430 (the compiler's wait for any shared-memory read then waits for them too), by asynchronous copies
+// 320, those two entries deep instead of one 223; flags precomputed by the rank kernel and the entries unrolled by
+// four (no register moves) 410 -> 320; rare paths (a revisit, a wait) in one branch each 237 -> 226.  Passes, first
+// build -> this one: 815 -> 467 us a wave (N_c = 1024), 3620 -> 1843 (N_c = 128, 65,536 droplets), 7007 -> 3697
+// (a window of 389^2).
 template <bool ECAP, bool LAKE>
-__global__ void __launch_bounds__(APPLY_THREADS, PGE_APPLY_MINB) ordered_apply_kernel(const OrderedArgs a)
+__global__ void __launch_bounds__(32) ordered_apply_kernel(const OrderedArgs a)
 {
-    __shared__ unsigned long long sstat[OS_N];
-    extern __shared__ Slot ring[];  // per droplet lane: RING slots
-    for (int k = threadIdx.x; k < OS_N; k += blockDim.x) sstat[k] = 0ull;
-    __syncthreads();
+    __shared__ EntryRec rec[REC_RING];
+    __shared__ alignas(16) ulonglong2 land[2][4];
+    __shared__ double hist[APPLY_HIST];  // the net change each of the last entries left at its cell
+    __shared__ double amt[32];           // what each entry of the chunk moved
+    __shared__ double capv[ECAP ? REC_RING : 1];
+    __shared__ float2 route[LAKE ? REC_RING : 1];
     const PgeParams &p = a.p;
-    // a.lanes droplets per warp, one per lane (1 when a pass runs alone: lanes of one warp that wait
-    // on different hand-offs take turns; more when other passes share the GPU, to hold fewer warps).
-    // A lane only ever waits for earlier droplets, which independent thread scheduling lets run.
-    const int lane = threadIdx.x & 31, lanes = a.lanes;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    Slot *R = ring + ((size_t)(threadIdx.x >> 5) * lanes + lane) * RING;
-    bool failed = false;
-    for (long long q = gw * lanes + lane; lane < lanes && !failed && q < a.nw; q += nwarps * lanes) {
-        const int K = (int)a.count[q];
-        if (K <= 0) {
-            a.dth[q] = -1;
-            continue;
-        }
-        const long long b0 = q * a.cap;
-        // prologue: the descriptors of the first DESC_AHEAD entries, then the cell data of the first CELL_AHEAD
-        for (int j = 0; j < DESC_AHEAD && j < K; j++) stage_desc(a, R[j], b0 + j);
-        cp_commit();
-        cp_wait<0>();
-        for (int j = 0; j < CELL_AHEAD && j < K; j++) stage_cell<ECAP, LAKE>(a, R[j]);
-        cp_commit();
-        cp_wait<0>();
-        Walk w;
-        w.deficit = w.surplus = w.prev_live = w.acc_c = 0.0;
-        w.clamped = 0;
-        w.death = -1;
-        w.w1c = w.w2c = w.w3c = -1;
-        w.w1v = w.w2v = w.w3v = 0.0;
-        w.sub_death = w.has_prev = w.have_c = false;
-        w.ok = true;
-        // the hand-off words are read into registers one entry ahead of the entry that first reads them
-        // (the terrain three ahead, through the ring): a word read later is less often stale
-        unsigned long long p0 = 0ull, p1 = 0ull;
-        Ent cur = load_ent<ECAP, LAKE>(R[0]);
-        hand_load_ahead(a.hand + cur.c, cur.h0, cur.h1);
-        if (K > 1) hand_load_ahead(a.hand + R[1].d.cell, p0, p1);
-        for (int k = 0; k < K; k++) {
-            // the copies issued LOOKAHEAD + 1 or more entries ago have landed: the descriptor of entry
-            // k + CELL_AHEAD and the cell data of entries k and k + 1
-            cp_wait<LOOKAHEAD>();
-            const bool has_next = k + 1 < K;
-            Ent nx;
-            nx.c = -1;
-            if (has_next) {
-                nx = load_ent<ECAP, LAKE>(R[(k + 1) & (RING - 1)]);
-                nx.h0 = p0;
-                nx.h1 = p1;
-            }
-            // entry k + 2's descriptor landed with the group waited for above
-            if (k + 2 < K) hand_load_ahead(a.hand + R[(k + 2) & (RING - 1)].d.cell, p0, p1);
-            if (k + CELL_AHEAD < K) stage_cell<ECAP, LAKE>(a, R[(k + CELL_AHEAD) & (RING - 1)]);
-            if (k + DESC_AHEAD < K) stage_desc(a, R[(k + DESC_AHEAD) & (RING - 1)], b0 + k + DESC_AHEAD);
-            cp_commit();
-            const int32_t c = cur.c;
-            const uint32_t df = cur.df;
-            const double dlt = cur.dlt;
-            const double hs = cur.hs;
-            const double b_c = (double)cur.base;
-            const bool park = (df & ENTRY_PARK) != 0;  // a lake park changes no terrain (particle.py:912-933)
-            const bool act = cur.active != 0 && !park;
-            if (!w.have_c && !(w.ok = cell_value(a, w, c, df, cur.h0, cur.h1, w.acc_c))) break;
-            // an erosion entry (floor) and a final deposit (ceiling) read the next entry's cell live:
-            // acquire it now; a step deposit does not, and acquires it only before writing it
-            const bool is_step = (df & ENTRY_STEP) != 0;
-            const bool reads_next = has_next && !park && (dlt < 0.0 || !is_step);
-            const int32_t ncell = nx.c;
-            double acc_n = 0.0, hs_n = 0.0;
-            if (reads_next) {
-                hs_n = nx.hs;
-                if (ncell == c)
-                    acc_n = w.acc_c;
-                else if (!(w.ok = cell_value(a, w, ncell, nx.df, nx.h0, nx.h1, acc_n)))
-                    break;
-            }
-            const double acc = w.acc_c;
-            double acc_new = acc, amount = 0.0;
-            entry_arith<ECAP, LAKE>(p, w, c, dlt, is_step, act, hs, b_c, acc, has_next, hs_n + acc_n, cur.cap, cur.route, acc_new,
-                                    amount);
-            // publish the net change; a droplet's last write at a cell also hands the cell on
-            const bool lastv = (df & ENTRY_LAST) != 0;
-            if (act || lastv) hand_store(a.hand + c, acc_new, a.epoch + (df & ENTRY_D_MASK) + (lastv ? 1u : 0u));
-            a.act[b0 + k] = amount;
-            w.w3c = w.w2c;
-            w.w3v = w.w2v;
-            w.w2c = w.w1c;
-            w.w2v = w.w1v;
-            w.w1c = c;
-            w.w1v = acc_new;
-            // the next entry's cell: acquired (with its net change) if this entry read it; the same
-            // cell again keeps its acquisition and its updated net change
-            if (has_next && ncell == c) {
-                w.have_c = true;
-                w.acc_c = acc_new;
-            } else {
-                w.have_c = reads_next;
-                w.acc_c = acc_n;
-            }
-            cur = nx;
-        }
-        cp_wait<0>();
-        if (!w.ok) {
-            failed = true;
-            break;
-        }
-        droplet_end(a, w, q, sstat);
+    const int lane = threadIdx.x;
+    const long long q = blockIdx.x;
+    const int K = (int)a.count[q];
+    if (K <= 0) {
+        if (lane == 0) a.dth[q] = -1;
+        return;
     }
-    __syncthreads();
-    flush_stats(a, sstat);
+    const EntryRec *list = a.rec + q * a.cap;
+    auto stage_rec = [&](int e) {
+        EntryRec *r = &rec[e & (REC_RING - 1)];
+        if (e < K) {
+            cp_cg16(r, list + e);
+            cp_cg16(reinterpret_cast<char *>(r) + 16, reinterpret_cast<const char *>(list + e) + 16);
+        } else {  // past the list's end: an entry that does nothing
+            r->flags = ENTRY_OPEN | ENTRY_FIRST | ENTRY_HELD;
+            r->cell = 0;
+        }
+    };
+    auto stage_ext = [&](int e) {  // an entry whose record has landed
+        if ((ECAP || LAKE) && e < K) {
+            const int32_t c = rec[e & (REC_RING - 1)].cell;
+            if (ECAP) cp_ca8(&capv[e & (REC_RING - 1)], a.ecap + c);
+            if (LAKE) cp_ca8(&route[e & (REC_RING - 1)], a.R + c);
+        }
+    };
+    stage_rec(lane);
+    stage_rec(32 + lane);
+    cp_commit();
+    cp_wait<0>();
+    __syncwarp();
+    stage_ext(lane);
+    EntryRec e0 = rec[0], e1 = rec[1], e2 = rec[2], e3 = rec[3];
+    // The hand-off words of the cells ahead: every entry sends for the words of the three after it, which land two
+    // entries on (a read of L2 takes as long as an entry); entry e's at e % 4, the sends of even and odd entries apart.
+    auto send = [&](int half, int at, int32_t c0, int32_t c1, int32_t c2) {
+        const int32_t c = lane == 0 ? c0 : lane == 1 ? c1 : c2;
+        __syncwarp();  // every lane has read what the words before these left there
+        if (lane < 3) cp_cg16(&land[half][(at + lane) & 3], a.hand + c);
+        cp_commit();
+    };
+    send(1, 0, e0.cell, e1.cell, e2.cell);
+    stage_rec(64 + lane);
+    cp_commit();
+    cp_wait<0>();
+    __syncwarp();
+    stage_ext(32 + lane);
+    ulonglong2 wa = land[1][0], wb = land[1][1];  // this entry's word and the next one's, as last read
+
+    Walk w;
+    w.deficit = w.surplus = 0.0;
+    w.prev_live = __longlong_as_double(0x7ff0000000000000ll);
+    w.clamped = 0;
+    w.death = -1;
+    w.sub_death = false;
+    long long eroded = 0, deposited = 0;
+    double held = 0.0;  // the net change of the current entry's cell, where the entry before it read it (ENTRY_HELD)
+    int k = 0;
+
+    // entry k + J (A) and the three after it; the record of entry k + J + 4 takes A's place
+    auto entry = [&](auto J_, EntryRec &A, const EntryRec &B, const EntryRec &C, const EntryRec &D) -> bool {
+        constexpr int J = decltype(J_)::value;
+        const uint32_t f = A.flags;
+        // the cell's net change, and where this entry needs the next one's cell that one's: a revisit takes what this
+        // droplet's own last visit left, else the earlier droplets have to have handed the cell on
+        const bool need_a = !(f & (ENTRY_HELD | ENTRY_OPEN)), need_b = (f & ENTRY_NEEDS) && !(B.flags & ENTRY_OPEN);
+        bool ok = (!need_a || hand_ready(wa.x, wa.y, A.turn)) && (!need_b || hand_ready(wb.x, wb.y, B.turn));
+        ulonglong2 wc;
+        const bool late = !ok;
+        if (late) {
+            for (int i = 0; !ok; i++) {
+                if (need_a && !hand_ready(wa.x, wa.y, A.turn)) hand_load(a.hand + A.cell, wa.x, wa.y);
+                hand_load(a.hand + B.cell, wb.x, wb.y);
+                hand_load(a.hand + C.cell, wc.x, wc.y);
+                const bool ok_a = !need_a || hand_ready(wa.x, wa.y, A.turn);
+                ok = ok_a && (!need_b || hand_ready(wb.x, wb.y, B.turn));
+                if ((i & 3) == 3 && !ok) {
+                    // droplets still to come before the one that hands the cell to this one: look less often, so that the
+                    // waiting warps leave their issue slots to the ones at work
+                    const uint32_t at = (uint32_t)((ok_a ? wb.x : wa.x) >> 32), want = ok_a ? B.turn : A.turn;
+                    const uint32_t away = want - ((int32_t)(at - a.epoch) < 0 ? a.epoch : at);
+                    if (away > 1) __nanosleep((away < PGE_BACK_MAX ? away - 1 : PGE_BACK_MAX) * PGE_BACK_NS);
+                    if ((i & (PGE_POLL_EVERY - 1)) == PGE_POLL_EVERY - 1 && (i >= kSpinLimit || *(volatile int *)a.error)) {
+                        if (i >= kSpinLimit) atomicExch(a.error, 1);
+                        return false;  // this wait, or another one, gave up
+                    }
+                }
+            }
+        }
+        send(J & 1, J + 1, B.cell, C.cell, D.cell);
+        double acc = (f & ENTRY_HELD) ? held : hand_acc(wa.x, wa.y), acc_n = hand_acc(wb.x, wb.y);
+        const bool again_a = !(f & (ENTRY_HELD | ENTRY_FIRST)), again_b = (f & ENTRY_NEEDS) && !(B.flags & ENTRY_FIRST);
+        if (again_a || again_b) {
+            auto own = [&](const EntryRec &r, int e) {
+                const int back = (int)(r.flags & ENTRY_BACK_MASK);
+                return back < APPLY_HIST ? hist[(e - back) & (APPLY_HIST - 1)] : own_value(a.hand, r.cell);
+            };
+            if (again_a) acc = own(A, k + J);
+            if (again_b) acc_n = own(B, k + J + 1);
+        }
+        acc_n = (f & ENTRY_SAME) ? acc : acc_n;
+        double moved;
+        const double acc_new = entry_arith<ECAP, LAKE>(p, w, A, acc, B.hs + acc_n, ECAP ? capv[(k & (REC_RING - 1)) + J] : 0.0,
+                                                       LAKE ? route[(k & (REC_RING - 1)) + J] : make_float2(0.f, 0.f), moved);
+        // a droplet's last write at a cell hands the cell on; before a revisit too far back for `hist` the net change is
+        // only left in the word
+        if ((f & (ENTRY_LAST | ENTRY_FAR)) && lane == 0) hand_store(a.hand + A.cell, acc_new, A.turn + ((f & ENTRY_LAST) ? 1u : 0u));
+        hist[(k & (APPLY_HIST - 1)) + J] = acc_new;
+        amt[(k & 31) + J] = moved;
+        held = (f & ENTRY_SAME) ? acc_new : acc_n;
+        A = rec[((k + 4) & (REC_RING - 1)) + J];
+        cp_wait<1>();
+        __syncwarp();
+        wa = land[(J + 1) & 1][(J + 1) & 3];
+        wb = late ? wc : land[(J + 1) & 1][(J + 2) & 3];
+        return true;
+    };
+    bool ok = true;
+    while (k < K) {
+        const int c0 = k, end = k + 32 < K ? k + 32 : K;
+        // (entries past the list's end do nothing)
+        for (; k < end; k += 4)
+            if (!(ok = entry(Int<0>{}, e0, e1, e2, e3) && entry(Int<1>{}, e1, e2, e3, e0) && entry(Int<2>{}, e2, e3, e0, e1) &&
+                       entry(Int<3>{}, e3, e0, e1, e2)))
+                break;
+        if (!ok) break;
+        // the chunk's statistics, and the records of the chunk two on (the next one's have landed)
+        __syncwarp();
+        if (c0 + lane < end) {
+            const double x = amt[lane];
+            if (signbit(x))
+                eroded += fx_mass(-x);
+            else
+                deposited += fx_mass(x);
+        }
+        cp_wait<0>();
+        __syncwarp();
+        stage_rec(k + 64 + lane);
+        stage_ext(k + 32 + lane);
+        cp_commit();
+    }
+    cp_wait<0>();
+    for (int o = 16; o > 0; o >>= 1) {
+        eroded += __shfl_xor_sync(FULL, eroded, o);
+        deposited += __shfl_xor_sync(FULL, deposited, o);
+    }
+    if (ok && lane == 0) droplet_end(a, w, q, eroded, deposited);
 }
 
 // ---------------------------------------------------------------------------
@@ -712,9 +657,7 @@ __global__ void ordered_gather_kernel(const OrderedArgs a, long long nslots, con
         g.v[i] = track ? v : 0.0f;
         g.m0[i] = track ? a.mom[2 * (long long)s] : 0.0f;
         g.m1[i] = track ? a.mom[2 * (long long)s + 1] : 0.0f;
-        const double amt = a.act[s];
-        g.amt[i] = a.delta[s] < 0.0 ? -amt : amt;  // the sign says erosion (an eroded 0 is -0)
-        g.kp[i] = (a.desc[s].dflags & ENTRY_LAST) && a.dth[q] == (int32_t)key ? a.keep[q] : -1.0;  // keep >= 0
+        g.kp[i] = (a.rec[s].flags & ENTRY_LAST) && a.dth[q] == (int32_t)key ? a.keep[q] : -1.0;  // keep >= 0
     }
 }
 
@@ -726,18 +669,14 @@ constexpr int FINISH_THREADS = 256, FINISH_WARPS = FINISH_THREADS / 32;
 __global__ void __launch_bounds__(FINISH_THREADS) ordered_finish_kernel(const OrderedArgs a, long long nslots, const unsigned long long *keys,
                                       unsigned long long invalid, FinishRows g)
 {
-    __shared__ unsigned long long sfx[2];
     // each warp's window of its run, read in order by every lane (broadcast reads: the loads of later slots
     // go out ahead of the float64 sums, which keep the serial order)
     __shared__ float sv[FINISH_WARPS][32], sa[FINISH_WARPS][32], sb[FINISH_WARPS][32];
     __shared__ double sk[FINISH_WARPS][32];
-    if (threadIdx.x < 2) sfx[threadIdx.x] = 0ull;
-    __syncthreads();
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    long long eroded = 0, deposited = 0;
     for (long long base = warp * 32; base < nslots; base += nwarps * 32) {
         const long long i = base + lane;
         const unsigned long long ki = i < nslots ? keys[i] : invalid;
@@ -760,11 +699,6 @@ __global__ void __launch_bounds__(FINISH_THREADS) ordered_finish_kernel(const Or
                     m0 = g.m0[j];
                     m1 = g.m1[j];
                     kp = g.kp[j];
-                    const double x = g.amt[j];
-                    if (signbit(x))
-                        eroded += fx_mass(-x);
-                    else
-                        deposited += fx_mass(x);
                 }
                 // the run covers a prefix of the lanes (keys are sorted)
                 const int n = __popc(__ballot_sync(full, in));
@@ -808,11 +742,6 @@ __global__ void __launch_bounds__(FINISH_THREADS) ordered_finish_kernel(const Or
             }
         }
     }
-    if (eroded) atomicAdd(&sfx[0], (unsigned long long)eroded);
-    if (deposited) atomicAdd(&sfx[1], (unsigned long long)deposited);
-    __syncthreads();
-    if (threadIdx.x == 0 && sfx[0]) red_add(reinterpret_cast<long long *>(&a.stats->eroded_fx), (long long)sfx[0]);
-    if (threadIdx.x == 1 && sfx[1]) red_add(reinterpret_cast<long long *>(&a.stats->deposited_fx), (long long)sfx[1]);
 }
 
 // zero the hand-off counters (the live net changes stay), so the 32-bit epochs can start over
@@ -835,14 +764,6 @@ cudaError_t ordered_terrain(long long ncell, const double2 *L, const float4 *B, 
 {
     ordered_terrain_kernel<<<grid_for(ncell), 256, 0, st>>>(ncell, L, B, mask, terr);
     return cudaPeekAtLastError();
-}
-
-int ordered_blocks_per_sm(int lanes)
-{
-    int n = 0;
-    const size_t smem = (size_t)(APPLY_THREADS / 32) * lanes * RING * sizeof(Slot);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ordered_apply_kernel<false, false>, APPLY_THREADS, smem) != cudaSuccess) return 1;
-    return n > 0 ? n : 1;
 }
 
 cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st)
@@ -873,27 +794,23 @@ cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st)
     tb = w.temp_bytes;
     if ((e = cub::DeviceScan::InclusiveScan(w.temp, tb, w.segpos, w.segscan, MaxOp{}, (int)nslots, st)) != cudaSuccess) return e;
     ordered_rank_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.keys_out, w.vals_out, w.cap, w.invalid, w.runscan, w.segscan,
-                                                          w.a.delta, w.a.vol, const_cast<EntryDesc *>(w.a.desc));
+                                                          w.a.delta, w.a.vol, w.a.count, w.a.terr, w.a.epoch, const_cast<EntryRec *>(w.a.rec));
     const bool lake = w.a.lakes && w.a.R;
-    const long long warps = (w.nw + w.a.lanes - 1) / w.a.lanes;  // a lane per droplet
-    long long blocks = (warps * 32 + APPLY_THREADS - 1) / APPLY_THREADS;
-    if (blocks > w.max_blocks) blocks = w.max_blocks;
-    const size_t smem = (size_t)(APPLY_THREADS / 32) * w.a.lanes * RING * sizeof(Slot);
+    const int blocks = (int)w.nw;  // a warp per droplet, the earlier droplets' blocks first
     if (w.a.ecap && lake)
-        ordered_apply_kernel<true, true><<<(int)blocks, APPLY_THREADS, smem, st>>>(w.a);
+        ordered_apply_kernel<true, true><<<blocks, 32, 0, st>>>(w.a);
     else if (w.a.ecap)
-        ordered_apply_kernel<true, false><<<(int)blocks, APPLY_THREADS, smem, st>>>(w.a);
+        ordered_apply_kernel<true, false><<<blocks, 32, 0, st>>>(w.a);
     else if (lake)
-        ordered_apply_kernel<false, true><<<(int)blocks, APPLY_THREADS, smem, st>>>(w.a);
+        ordered_apply_kernel<false, true><<<blocks, 32, 0, st>>>(w.a);
     else
-        ordered_apply_kernel<false, false><<<(int)blocks, APPLY_THREADS, smem, st>>>(w.a);
+        ordered_apply_kernel<false, false><<<blocks, 32, 0, st>>>(w.a);
     // the sort's input keys and the scans' buffers are free again: the gathered rows live there
     FinishRows g;
     g.v = reinterpret_cast<float *>(w.runstart);
     g.m0 = reinterpret_cast<float *>(w.segpos);
     g.m1 = reinterpret_cast<float *>(w.runscan);
-    g.amt = reinterpret_cast<double *>(w.keys_in);
-    g.kp = w.fin_kp;
+    g.kp = reinterpret_cast<double *>(w.keys_in);
     ordered_gather_kernel<<<grid_for(nslots), 256, 0, st>>>(w.a, nslots, w.keys_out, w.vals_out, w.invalid, g);
     ordered_finish_kernel<<<grid_for(nslots, FINISH_THREADS), FINISH_THREADS, 0, st>>>(w.a, nslots, w.keys_out, w.invalid, g);
     return cudaPeekAtLastError();

@@ -4,17 +4,32 @@
 
 namespace pge {
 
-// one entry of a wave's change lists as the ordered apply reads it (built by the rank kernel)
-struct alignas(16) EntryDesc {
-    int32_t cell;
-    uint32_t dflags;  // D (distinct earlier droplets of the wave at the cell) | ENTRY_* flags
+// one entry of a wave's change lists as the ordered apply reads it (built by the rank kernel): the entry, its
+// cell's read-only terrain and where its droplet was there before, so that the apply reads nothing else but the
+// hand-off words
+struct alignas(16) EntryRec {
     double delta;
+    double hs;       // height + sediment at the start of the pass
+    float base;
+    uint32_t flags;  // ENTRY_* | entries since its droplet's previous visit to the cell (0: none; APPLY_HIST: that or more)
+    int32_t cell;
+    uint32_t turn;   // the cell's hand-off counter once the earlier droplets of the wave have handed it on
 };
-constexpr uint32_t ENTRY_D_MASK = 0xffffffu;
-constexpr uint32_t ENTRY_LAST = 1u << 24;   // its droplet's last visit to the cell
-constexpr uint32_t ENTRY_FIRST = 1u << 25;  // its droplet's first visit to the cell
-constexpr uint32_t ENTRY_STEP = 1u << 26;   // a step entry (vol >= 0), not a final deposit
-constexpr uint32_t ENTRY_PARK = 1u << 27;   // a lake park (vol -3): its cell is visited and handed on unchanged
+static_assert(sizeof(EntryRec) == 32, "two 16-byte reads an entry");
+// entries whose net change the apply keeps on chip for its droplet's own revisits
+constexpr int APPLY_HIST = 128;
+constexpr uint32_t ENTRY_BACK_MASK = 0xffu;
+constexpr uint32_t ENTRY_LAST = 1u << 8;    // its droplet's last visit to the cell
+constexpr uint32_t ENTRY_FIRST = 1u << 9;   // its droplet's first visit to the cell
+constexpr uint32_t ENTRY_OPEN = 1u << 10;   // no earlier droplet to wait for: a revisit, or the wave's first visitor
+constexpr uint32_t ENTRY_STEP = 1u << 11;   // a step entry (vol >= 0), not a bank cut, a park or a final deposit
+constexpr uint32_t ENTRY_DEP = 1u << 12;    // deposits (delta >= 0) on an active cell
+constexpr uint32_t ENTRY_ERO = 1u << 13;    // erodes (delta < 0) an active cell; neither: changes nothing (a lake park among them)
+constexpr uint32_t ENTRY_READS = 1u << 14;  // reads the next entry's cell: an erosion's floor, a final deposit's ceiling
+constexpr uint32_t ENTRY_NEEDS = 1u << 15;  // reads it, and it is another cell
+constexpr uint32_t ENTRY_SAME = 1u << 16;   // the next entry is at the same cell
+constexpr uint32_t ENTRY_HELD = 1u << 17;   // the entry before it read this cell, or is at it: its net change is at hand
+constexpr uint32_t ENTRY_FAR = 1u << 18;    // its droplet comes back only after APPLY_HIST entries or more
 
 // a cell's read-only terrain for the ordered apply (built once per pass)
 struct alignas(16) CellTerr {
@@ -32,7 +47,7 @@ struct OrderedArgs {
     const int64_t *count;
     int cap;
     long long nw;
-    const EntryDesc *desc;
+    const EntryRec *rec;
     const CellTerr *terr;
     // terrain
     const double2 *L;  // x: height + sediment
@@ -46,12 +61,9 @@ struct OrderedArgs {
     // per cell: the live net change and the hand-off counter, one 16-byte word
     double2 *hand;
     uint32_t epoch;  // this wave's: a cell with D earlier visitors is free once its counter reads epoch + D
-    int lanes;  // droplets per warp in the apply
     // per droplet: the stockpile cell (-1: none) and the amount it adds there
     int32_t *dth;
     double *keep;
-    // per slot: the amount the entry actually eroded or deposited (its statistics are summed later)
-    double *act;
     // float64 accumulators in serial order: (net change, discharge, momentum a, b) and the stockpile
     double *acc4;
     double *pend;
@@ -86,7 +98,6 @@ struct ParkWave {
 // what each sorted slot adds to its cell, gathered in sorted order for the finish
 struct FinishRows {
     float *v, *m0, *m1;  // step volume and momentum (0 unless a step of volume > 0 on an active cell)
-    double *amt;         // the amount applied, negative for an erosion entry
     double *kp;          // the droplet's stockpile where this is its last visit to its stockpile cell, else -1
 };
 
@@ -99,8 +110,6 @@ struct OrderedWave {
     int32_t *vals_in, *vals_out, *runstart, *segpos, *runscan, *segscan;
     void *temp;
     size_t temp_bytes;
-    long long max_blocks;
-    double *fin_kp;  // one double a slot: the gathered stockpile amounts
     // long lists: the recorded entries compacted before the ranks (nullptr: every slot goes through them);
     // max_wave + 1 int64: each droplet's first entry, then the wave's total
     long long *offsets;
@@ -114,7 +123,6 @@ constexpr int COMPACT_CAP = PGE_COMPACT_CAP;
 
 size_t ordered_temp_bytes(long long nslots, long long max_wave);
 cudaError_t park_wave(const ParkWave &pw, cudaStream_t st);
-int ordered_blocks_per_sm(int lanes);  // resident blocks of the apply kernel per SM
 cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st);
 cudaError_t hand_reset(long long ncell, double2 *hand, cudaStream_t st);
 cudaError_t ordered_terrain(long long ncell, const double2 *L, const float4 *B, const uint8_t *mask, CellTerr *terr, cudaStream_t st);
