@@ -417,8 +417,8 @@ PGE_API int pge_halo_gather(const PgeHalo *h, double *field, int32_t vector, voi
  * outside or halo cell; s->mask (may be NULL) excludes outside cells; owner is
  * the (F,NE,NE) int32 owner table (cubesphere.py:664-674; the identity for a
  * window).  Surface = s->height + s->sediment.  Runs a relaxation to its fixed
- * point, synchronising the stream every 32 sweeps to test it; *sweeps (host,
- * may be NULL) gets the sweeps run; PGE_E_UNSUPPORTED if max_sweeps did not
+ * point, a 32 x 32 tile at a time, synchronising the stream every 8 sweeps to
+ * test it; *sweeps (host, may be NULL) gets the sweeps run; PGE_E_UNSUPPORTED if max_sweeps did not
  * reach the fixed point. */
 PGE_API int pge_route_flood(const PgeGrid *g, const PgeState *s, const int32_t *owner, double eps, double *route, int64_t max_sweeps,
                             int64_t *sweeps, void *ws, size_t ws_bytes, void *stream);
@@ -436,8 +436,8 @@ PGE_API int pge_route_flood(const PgeGrid *g, const PgeState *s, const int32_t *
  * component, -1 above the waterline).  Components are joined along the
  * owner relation taken both ways (the reference walks it one way from each
  * component's lowest cell; they differ only where a cube corner's halo
- * mapping is one-sided).  Synchronises the stream every 16 sweeps; spherical
- * grids only. */
+ * mapping is one-sided).  One pass: *sweeps (host, may be NULL) gets 1;
+ * spherical grids only. */
 PGE_API int pge_sea_base(const PgeGrid *g, const PgeState *s, const int32_t *owner, const float *area, double min_area, double *base,
                          int32_t *labels, int64_t max_sweeps, int64_t *sweeps, void *ws, size_t ws_bytes, void *stream);
 

@@ -1287,10 +1287,9 @@ __global__ void route_init_kernel(int F, int NE, int H, int N, const double *__r
                                   const double *__restrict__ base, const uint8_t *__restrict__ mask, const int32_t *__restrict__ owner,
                                   unsigned long long *key, unsigned char *state)
 {
-    const long long total = (long long)F * NE * NE;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total; c += (long long)gridDim.x * blockDim.x) {
-        const int f = (int)(c / ((long long)NE * NE));
-        const int ei = (int)((c / NE) % NE), ej = (int)(c % NE);
+    const unsigned total = (unsigned)F * NE * NE;
+    for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < total; u += gridDim.x * blockDim.x) {
+        const int c = (int)u, r = c / NE, ej = c - r * NE, ei = r % NE;
         const double sv = h[c] + s[c];
         const bool outside = mask && mask[c] == PGE_MASK_OUTSIDE;
         if (outside || ei == 0 || ej == 0 || ei == NE - 1 || ej == NE - 1) {
@@ -1301,15 +1300,16 @@ __global__ void route_init_kernel(int F, int NE, int H, int N, const double *__r
         bool seed = false;
         if (ei >= H && ei < H + N && ej >= H && ej < H + N) {
             seed = sv < 0.0 && sv <= base[c];
-            for (int k = 0; k < 8 && !seed; k++) {
-                const long long n = owner[((long long)f * NE + ei + kRouteD8[k][0]) * NE + ej + kRouteD8[k][1]];
+            // a neighbour outside the mask, or none that is real (a window's edge): only beside the halo without a mask
+            const bool rim = mask || ei == H || ei == H + N - 1 || ej == H || ej == H + N - 1;
+            for (int k = 0; k < 8 && rim && !seed; k++) {
+                const int n = owner[c + kRouteD8[k][0] * NE + kRouteD8[k][1]];
                 if (mask && mask[n] == PGE_MASK_OUTSIDE) {
                     seed = true;
                     break;
                 }
-                const long long rem = n % ((long long)NE * NE);
-                const int nei = (int)(rem / NE), nej = (int)(rem % NE);
-                if (nei < H || nei >= H + N || nej < H || nej >= H + N) seed = true;  // no real neighbour (window edge)
+                const int nr = n / NE, nej = n - nr * NE, nei = nr % NE;
+                if (nei < H || nei >= H + N || nej < H || nej >= H + N) seed = true;
             }
         }
         state[c] = seed ? RF_SEED : RF_FREE;
@@ -1317,28 +1317,123 @@ __global__ void route_init_kernel(int F, int NE, int H, int N, const double *__r
     }
 }
 
-__global__ void route_push_kernel(int F, int NE, const double *__restrict__ h, const double *__restrict__ s, const int32_t *__restrict__ owner,
-                                  double eps, unsigned long long *key, const unsigned char *__restrict__ state,
-                                  unsigned long long *changed)
+// One sweep of the relaxation, a tile a block: every active tile is relaxed to its own fixed point in shared memory
+// (a cell takes what its lowest neighbour gives it), written back, and the tiles that its changed cells can lower
+// are made active for the next sweep.  Within a face a cell's neighbours push to it what it pulls here; across a
+// cube edge (the neighbour is a halo cell, owned by an interior cell of another face) the push goes to the owner.
+// The values only ever fall, to the one fixed point, so neither the order nor a stale neighbour changes the result.
+//
+// Bound by the relaxations inside the tiles.  N_c = 1024, evolved world: sweeps of every cell from HBM, one cell
+// further a sweep, 384 x 112 us; tiles, 16 sweeps of what is active, 66 us each.
+constexpr int RT = 32;         // tile edge
+constexpr int RT_STRIP = 4;    // cells a thread, one above the other
+constexpr int RT_ROUNDS = 2;   // relaxations between two looks at whether the tile still changes
+__global__ void __launch_bounds__(RT *RT / RT_STRIP) route_tile_kernel(int NE, int H, int tiles, const double *__restrict__ h,
+                                                                       const double *__restrict__ s, const int32_t *__restrict__ owner,
+                                                                       double eps, unsigned long long *key,
+                                                                       const unsigned char *__restrict__ state, int first, int *active,
+                                                                       int *next, unsigned long long *changed)
 {
-    const long long total = (long long)F * NE * NE;
-    bool any = false;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total; c += (long long)gridDim.x * blockDim.x) {
-        if (state[c] == RF_EXCLUDED) continue;
-        const unsigned long long kc = ((volatile unsigned long long *)key)[c];
-        if (kc == RF_UNREACHED) continue;
-        const double v = unokey(kc) + eps;
-        const int f = (int)(c / ((long long)NE * NE));
-        const int ei = (int)((c / NE) % NE), ej = (int)(c % NE);
-        for (int k = 0; k < 8; k++) {
-            const long long n = owner[((long long)f * NE + ei + kRouteD8[k][0]) * NE + ej + kRouteD8[k][1]];
+    __shared__ unsigned long long sk[RT + 2][RT + 2];
+    const int tile = blockIdx.x;
+    if (!__syncthreads_or(first || active[tile])) return;  // (one look for the whole block: the flag is cleared below)
+    const int f = tile / (tiles * tiles), tr = tile - f * tiles * tiles, ti = tr / tiles, tj = tr - ti * tiles;
+    const int fb = f * NE * NE, i0 = ti * RT, j0 = tj * RT;
+    const int tx = threadIdx.x % RT, ty = threadIdx.x / RT;
+    const volatile unsigned long long *vkey = key;
+    // a cell that takes part: not excluded, and its own owner (a halo cell of the sphere only stands for another)
+    for (int q = threadIdx.x; q < (RT + 2) * (RT + 2); q += blockDim.x) {
+        const int a = q / (RT + 2), b = q - a * (RT + 2), i = i0 + a - 1, j = j0 + b - 1;
+        unsigned long long k = RF_UNREACHED;
+        if (i >= 0 && i < NE && j >= 0 && j < NE) {
+            const int c = fb + i * NE + j;
+            if (state[c] != RF_EXCLUDED && owner[c] == c) k = vkey[c];
+        }
+        sk[a][b] = k;
+    }
+    if (threadIdx.x == 0 && !first) active[tile] = 0;
+    double surf[RT_STRIP];
+    unsigned long long was[RT_STRIP];
+    bool free_[RT_STRIP], in[RT_STRIP];
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RT_STRIP; r++) {
+        const int i = i0 + ty * RT_STRIP + r, j = j0 + tx;
+        in[r] = i < NE && j < NE;
+        free_[r] = false;
+        surf[r] = 0.0;
+        was[r] = sk[ty * RT_STRIP + r + 1][tx + 1];
+        if (in[r]) {
+            const int c = fb + i * NE + j;
+            in[r] = owner[c] == c && state[c] != RF_EXCLUDED;
+            free_[r] = in[r] && state[c] == RF_FREE;
+            surf[r] = h[c] + s[c];
+        }
+    }
+    volatile unsigned long long(*vk)[RT + 2] = sk;
+    bool any = true;
+    while (any) {
+        bool mine = false;
+#pragma unroll
+        for (int t = 0; t < 2 * RT_ROUNDS; t++) {
+#pragma unroll
+            for (int q = 0; q < RT_STRIP; q++) {
+                const int r = t & 1 ? RT_STRIP - 1 - q : q;  // down the strip, then up
+                if (!free_[r]) continue;
+                const int a = ty * RT_STRIP + r + 1, b = tx + 1;
+                unsigned long long m = vk[a - 1][b - 1];
+                m = min(m, vk[a - 1][b]);
+                m = min(m, vk[a - 1][b + 1]);
+                m = min(m, vk[a][b - 1]);
+                m = min(m, vk[a][b + 1]);
+                m = min(m, vk[a + 1][b - 1]);
+                m = min(m, vk[a + 1][b]);
+                m = min(m, vk[a + 1][b + 1]);
+                if (m == RF_UNREACHED) continue;
+                const double v = unokey(m) + eps;
+                const unsigned long long kn = okey(surf[r] > v ? surf[r] : v);
+                if (kn < vk[a][b]) {
+                    vk[a][b] = kn;
+                    mine = true;
+                }
+            }
+        }
+        any = __syncthreads_or(mine);
+    }
+    // write back, push across the cube edges, and wake the tiles whose cells this tile's rim can still lower (whoever
+    // lowered the rim: this tile, or a push from another face since it last ran)
+    bool woke = false;
+#pragma unroll
+    for (int r = 0; r < RT_STRIP; r++) {
+        if (!in[r]) continue;
+        const int a = ty * RT_STRIP + r, b = tx, i = i0 + a, j = j0 + b, c = fb + i * NE + j;
+        const unsigned long long k = sk[a + 1][b + 1];
+        if (k == RF_UNREACHED) continue;
+        if (k < was[r]) atomicMin(key + c, k);
+        const bool rim = a == 0 || a == RT - 1 || b == 0 || b == RT - 1 || i == H || i == NE - H - 1 || j == H || j == NE - H - 1;
+        if (!rim) continue;
+        const double v = unokey(k) + eps;
+        for (int d = 0; d < 8; d++) {
+            const int di = kRouteD8[d][0], dj = kRouteD8[d][1], nc = c + di * NE + dj;  // (excluded cells ring the array)
+            const int n = owner[nc];
+            int nt;  // the neighbour's tile
+            if (n == nc) {
+                nt = (f * tiles + (i + di) / RT) * tiles + (j + dj) / RT;
+                if (nt == tile) continue;
+            } else {
+                const int nf = n / (NE * NE), nr = n - nf * NE * NE;
+                nt = (nf * tiles + nr / NE / RT) * tiles + nr % NE / RT;
+            }
             if (state[n] != RF_FREE) continue;
             const double sn = h[n] + s[n];
             const unsigned long long kn = okey(sn > v ? sn : v);
-            if (kn < ((volatile unsigned long long *)key)[n] && atomicMin(key + n, kn) > kn) any = true;
+            if (kn < vkey[n] && (n == nc || atomicMin(key + n, kn) > kn)) {
+                next[nt] = 1;
+                woke = true;
+            }
         }
     }
-    if (any) *changed = 1ull;
+    if (__syncthreads_or(woke) && threadIdx.x == 0) *changed = 1ull;
 }
 
 __global__ void route_final_kernel(long long total, const double *__restrict__ h, const double *__restrict__ s,
@@ -1358,15 +1453,22 @@ cudaError_t route_flood(const PgeGrid &g, const PgeState &st, const int32_t *own
     unsigned long long *key = ws_ptr<unsigned long long>(ws, lay.cdf);
     unsigned char *state = ws_ptr<unsigned char>(ws, lay.flags);
     unsigned long long *changed = ws_ptr<unsigned long long>(ws, lay.counters) + 8;
+    const int tiles = (NE + RT - 1) / RT, nt = g.F * tiles * tiles;
+    int *active = reinterpret_cast<int *>(state + (n + 7) / 8 * 8);  // two flags a tile, in the 7 bytes a cell left here
     route_init_kernel<<<grid_for(n), 256, 0, s>>>(g.F, NE, g.H, g.N, st.height, st.sediment, st.base, st.mask, owner, key, state);
+    cudaError_t e = cudaMemsetAsync(active, 0, 2 * sizeof(int) * nt, s);
+    if (e != cudaSuccess) return e;
     unsigned long long host_changed = 1;
     long long sweeps = 0;
-    const int batch = 32;  // sweeps between convergence checks (the check synchronises the stream)
+    const int batch = 8;  // sweeps between convergence checks (the check synchronises the stream)
     while (host_changed && sweeps < max_sweeps) {
-        cudaError_t e = cudaMemsetAsync(changed, 0, 8, s);
-        if (e != cudaSuccess) return e;
-        for (int k = 0; k < batch; k++)
-            route_push_kernel<<<grid_for(n), 256, 0, s>>>(g.F, NE, st.height, st.sediment, owner, eps, key, state, changed);
+        for (int k = 0; k < batch; k++) {
+            // (the last sweep of the batch says whether any tile is left to relax)
+            if ((e = cudaMemsetAsync(changed, 0, 8, s)) != cudaSuccess) return e;
+            const long long w = sweeps + k;
+            route_tile_kernel<<<nt, RT * RT / RT_STRIP, 0, s>>>(NE, g.H, tiles, st.height, st.sediment, owner, eps, key, state, w == 0,
+                                                                active + (w & 1) * nt, active + ((w + 1) & 1) * nt, changed);
+        }
         sweeps += batch;
         if ((e = cudaMemcpyAsync(&host_changed, changed, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
@@ -1380,71 +1482,159 @@ cudaError_t route_flood(const PgeGrid &g, const PgeState &st, const int32_t *own
 // sea mask: the base level (maps.py:360-420, hydro/run.py:64-83).  Interior
 // cells under the waterline (float32 surface < 0) are joined into
 // 8-connected components along the owner table (labels: the component's
-// lowest cell id, by min-label propagation with pointer jumping); a component
+// lowest cell id, by one pass of unions; propagating labels cell by cell took
+// 256 sweeps of 194 us for the oceans of N_c = 1024); a component
 // is open ocean when its area reaches min_area, and the largest always is;
 // the others are closed basins, whose cells take the basin's lowest surface.
 // ---------------------------------------------------------------------------
 namespace {
-__device__ __forceinline__ long long sea_ext(long long c, int N, int H, int NE)
+// the interior cell that owns neighbour k of interior cell c, or -1 where the owner table names a halo cell (a grid
+// too small for its halo's sources)
+__device__ __forceinline__ int sea_nb(const int32_t *owner, int c, int k, int N, int H, int NE)
 {
-    const long long f = c / ((long long)N * N), rem = c % ((long long)N * N);
-    return (f * NE + rem / N + H) * NE + rem % N + H;
-}
-__device__ __forceinline__ long long sea_nb(const int32_t *owner, long long c, int k, int N, int H, int NE)
-{
-    const long long f = c / ((long long)N * N), rem = c % ((long long)N * N);
-    const long long o = owner[(f * NE + rem / N + H + kRouteD8[k][0]) * NE + rem % N + H + kRouteD8[k][1]];
-    const long long f2 = o / ((long long)NE * NE), r2 = o % ((long long)NE * NE);
-    return (f2 * N + r2 / NE - H) * N + r2 % NE - H;
+    const int row = c / N, j = c - row * N, f = row / N, i = row - f * N;
+    const int o = owner[(f * NE + i + H + kRouteD8[k][0]) * NE + j + H + kRouteD8[k][1]];
+    const int orow = o / NE, oj = o - orow * NE - H, of = orow / NE, oi = orow - of * NE - H;
+    return oi < 0 || oi >= N || oj < 0 || oj >= N ? -1 : (of * N + oi) * N + oj;
 }
 }  // namespace
 
-__global__ void sea_init_kernel(long long M, int N, int H, int NE, const double *__restrict__ h, const double *__restrict__ s,
+// Components by union-find (N_c = 1024: 0.45 ms for the three passes): a label is the parent cell, a root its own, and unions point the larger root at the
+// smaller, so a component's root ends as its lowest cell id.  Each run of 32 cells of a row starts joined to its first.
+__device__ __forceinline__ int sea_find(int32_t *label, int c)
+{
+    volatile int32_t *l = label;
+    int p = l[c];
+    while (p != c) {  // halving the path: any ancestor is a valid parent
+        const int g = l[p];
+        if (g != p) l[c] = g;
+        c = p;
+        p = g;
+    }
+    return c;
+}
+
+__device__ __forceinline__ void sea_unite(int32_t *label, int a, int b)
+{
+    while (true) {
+        a = sea_find(label, a);
+        b = sea_find(label, b);
+        if (a == b) return;
+        if (a < b) {
+            const int t = a;
+            a = b;
+            b = t;
+        }
+        const int old = atomicMin(label + a, b);
+        if (old == a) return;
+        a = old;  // another union moved that root: join what it joined
+    }
+}
+
+__global__ void sea_init_kernel(int M, int N, int H, int NE, const double *__restrict__ h, const double *__restrict__ s,
                                 int32_t *label, double *per, unsigned long long *floorkey)
 {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < M; c += (long long)gridDim.x * blockDim.x) {
-        const long long e = sea_ext(c, N, H, NE);
-        label[c] = (float)(h[e] + s[e]) < 0.0f ? (int32_t)c : -1;
-        per[c] = 0.0;
-        floorkey[c] = okey(0.0);  // the basin floor starts at 0 (maps.py: np.zeros, then np.minimum.at)
+    const int lane = threadIdx.x & 31;
+    for (unsigned c0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; c0 < (unsigned)M; c0 += gridDim.x * blockDim.x) {
+        const int c = (int)c0 + lane;
+        const int row = c / N, j = c - row * N, f = row / N, i = row - f * N;
+        bool below = false;
+        if (c < M) {
+            const int e = (f * NE + i + H) * NE + j + H;
+            below = (float)(h[e] + s[e]) < 0.0f;
+        }
+        const unsigned land = ~__ballot_sync(0xffffffffu, below) & ((1u << lane) - 1u);
+        int start = land ? 32 - __clz(land) : 0;  // the run's first lane: after the last land cell, in this row
+        start = max(start, lane - j);
+        if (c < M) {
+            label[c] = below ? c - (lane - start) : -1;
+            per[c] = 0.0;
+            floorkey[c] = okey(0.0);  // the basin floor starts at 0 (maps.py: np.zeros, then np.minimum.at)
+        }
     }
 }
 
-__global__ void sea_join_kernel(long long M, int N, int H, int NE, const int32_t *__restrict__ owner, int32_t *label,
-                                unsigned long long *changed)
+__global__ void sea_join_kernel(int M, int N, int H, int NE, const int32_t *__restrict__ owner, int32_t *label)
 {
-    bool any = false;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < M; c += (long long)gridDim.x * blockDim.x) {
-        const int l = ((volatile int32_t *)label)[c];
-        if (l < 0) continue;
-        int m = l;
-        const int ll = ((volatile int32_t *)label)[l];  // pointer jumping: the label of the label
-        if (ll >= 0 && ll < m) m = ll;
-        long long nb[8];
-        for (int k = 0; k < 8; k++) {
-            nb[k] = sea_nb(owner, c, k, N, H, NE);
-            const int lq = ((volatile int32_t *)label)[nb[k]];
-            if (lq >= 0 && lq < m) m = lq;
-        }
-        if (m < l && atomicMin(label + c, m) > m) any = true;
-        for (int k = 0; k < 8; k++) {
-            const int lq = ((volatile int32_t *)label)[nb[k]];
-            if (lq > m && atomicMin(label + nb[k], m) > m) any = true;
+    for (unsigned u = blockIdx.x * blockDim.x + threadIdx.x; u < (unsigned)M; u += gridDim.x * blockDim.x) {
+        const int c = (int)u;
+        if (((volatile int32_t *)label)[c] < 0) continue;
+        const int row = c / N, j = c - row * N, i = row % N;
+        auto below = [&](int q) { return ((volatile int32_t *)label)[q] >= 0; };
+        if (i == 0 || i == N - 1 || j == 0 || j == N - 1) {  // beside the halo: along the owner table
+            for (int k = 0; k < 8; k++) {
+                const int q = sea_nb(owner, c, k, N, H, NE);
+                if (q >= 0 && below(q)) sea_unite(label, c, q);
+            }
+        } else {
+            // the row above joins itself, so one of its cells that touch is enough; a run joins the one left of it
+            if (below(c - N)) {
+                sea_unite(label, c, c - N);
+            } else {
+                if (below(c - N - 1)) sea_unite(label, c, c - N - 1);
+                if (below(c - N + 1)) sea_unite(label, c, c - N + 1);
+            }
+            if ((c & 31) == 0 && below(c - 1)) sea_unite(label, c, c - 1);
         }
     }
-    if (any) *changed = 1ull;
 }
 
-__global__ void sea_stats_kernel(long long M, int N, int H, int NE, const double *__restrict__ h, const double *__restrict__ s,
+// (the walk to the root halves no path here: a thread writes its own cell only, so what it writes stays)
+__global__ void sea_flatten_kernel(int M, int32_t *label)
+{
+    volatile int32_t *l = label;
+    for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < (unsigned)M; c += gridDim.x * blockDim.x) {
+        int r = l[c];
+        if (r < 0) continue;
+        while (l[r] != r) r = l[r];
+        l[c] = r;
+    }
+}
+
+// the area and the lowest surface of each component (two atomics a cell, all on the ocean's root: 6.8 ms at N_c = 1024;
+// as here 53 us): a thread keeps the sums of the label it is at, and a warp whose
+// lanes are all at one label (the open ocean nearly everywhere) adds its sum once
+constexpr int SEA_PER_LANE = 16;
+__global__ void sea_stats_kernel(int M, int N, int H, int NE, const double *__restrict__ h, const double *__restrict__ s,
                                  const float *__restrict__ area, const int32_t *__restrict__ label, double *per,
                                  unsigned long long *floorkey)
 {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < M; c += (long long)gridDim.x * blockDim.x) {
-        const int l = label[c];
-        if (l < 0) continue;
-        const long long e = sea_ext(c, N, H, NE);
-        atomicAdd(per + l, (double)area[c]);
-        atomicMin(floorkey + l, okey(h[e] + s[e]));
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int w0 = warp; w0 < (M + 32 * SEA_PER_LANE - 1) / (32 * SEA_PER_LANE); w0 += nwarps) {
+        int lab = -1;
+        double sum = 0.0;
+        unsigned long long low = RF_UNREACHED;
+        auto flush = [&]() {
+            if (lab < 0) return;
+            atomicAdd(per + lab, sum);
+            atomicMin(floorkey + lab, low);
+        };
+        for (int t = 0; t < SEA_PER_LANE; t++) {
+            const int c = (w0 * SEA_PER_LANE + t) * 32 + lane;
+            const int l = c < M ? label[c] : -1;
+            if (l < 0) continue;
+            if (l != lab) {
+                flush();
+                lab = l;
+                sum = 0.0;
+                low = RF_UNREACHED;
+            }
+            const int row = c / N, j = c - row * N, f = row / N, i = row - f * N, e = (f * NE + i + H) * NE + j + H;
+            sum += (double)area[c];
+            low = min(low, okey(h[e] + s[e]));
+        }
+        const int l0 = __reduce_max_sync(full, lab);
+        if (__all_sync(full, lab == l0 || lab < 0)) {
+            for (int o = 16; o > 0; o >>= 1) {
+                sum += __shfl_xor_sync(full, sum, o);
+                low = min(low, __shfl_xor_sync(full, low, o));
+            }
+            lab = l0;
+            if (lane == 0) flush();
+        } else {
+            flush();
+        }
     }
 }
 
@@ -1485,20 +1675,14 @@ cudaError_t sea_base(const PgeGrid &g, const PgeState &st, const int32_t *owner,
     double *per = ws_ptr<double>(ws, lay.cdf);
     unsigned long long *floorkey = reinterpret_cast<unsigned long long *>(per + M);
     unsigned long long *cnt = ws_ptr<unsigned long long>(ws, lay.counters);
-    unsigned long long *changed = cnt + 9, *maxkey = cnt + 10, *largest = cnt + 11;
-    sea_init_kernel<<<grid_for(M), 256, 0, s>>>(M, N, H, NE, st.height, st.sediment, label, per, floorkey);
-    unsigned long long host_changed = 1;
-    long long sweeps = 0;
+    unsigned long long *maxkey = cnt + 10, *largest = cnt + 11;
+    const int m = (int)M;  // (check_shape: the cells count in int32)
+    sea_init_kernel<<<grid_for(M), 256, 0, s>>>(m, N, H, NE, st.height, st.sediment, label, per, floorkey);
+    sea_join_kernel<<<grid_for(M), 256, 0, s>>>(m, N, H, NE, owner, label);
+    sea_flatten_kernel<<<grid_for(M), 256, 0, s>>>(m, label);
+    if (sweeps_out) *sweeps_out = 1;
+    sea_stats_kernel<<<grid_reduce(M / SEA_PER_LANE + 1), 256, 0, s>>>(m, N, H, NE, st.height, st.sediment, area, label, per, floorkey);
     cudaError_t e;
-    while (host_changed && sweeps < max_sweeps) {
-        if ((e = cudaMemsetAsync(changed, 0, 8, s)) != cudaSuccess) return e;
-        for (int k = 0; k < 16; k++) sea_join_kernel<<<grid_for(M), 256, 0, s>>>(M, N, H, NE, owner, label, changed);
-        sweeps += 16;
-        if ((e = cudaMemcpyAsync(&host_changed, changed, 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess) return e;
-        if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return e;
-    }
-    if (sweeps_out) *sweeps_out = host_changed ? -sweeps : sweeps;
-    sea_stats_kernel<<<grid_for(M), 256, 0, s>>>(M, N, H, NE, st.height, st.sediment, area, label, per, floorkey);
     if ((e = cudaMemsetAsync(maxkey, 0, 8, s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(largest, 0xFF, 8, s)) != cudaSuccess) return e;
     sea_largest_kernel<<<grid_for(M), 256, 0, s>>>(M, label, per, maxkey, largest, 0);
