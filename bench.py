@@ -308,7 +308,7 @@ def launches_per_iteration(nw: int, pending: bool, creep: bool, ordered: bool) -
         droplets = 3 + 7 * nw + 3
     else:         # pack x2; waves and the refreshes between them; mode, fold+EMA
         droplets = 2 + nw + (nw - 1) + 2
-    thermal = 4 * (2 if creep else 1)
+    thermal = 2  # the talus pass, then the creep pass or the copy back
     uplift = 4    # the mean's pairwise sum (plan, leaves, fold), the add
     datum = 1 + 8 * 2 + 1
     halo = 4

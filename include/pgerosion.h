@@ -635,7 +635,7 @@ PGE_API int pge_crmath_host(int32_t op, int64_t n, const double *x, double *y);
  * allocate device memory -- a host that owns the whole device heap through
  * its own pool and forbids other allocations, or a loop that must not pay
  * cudaMalloc's latency and implicit synchronisation: no workspace, the
- * scratch is a static device array of PGE_NOALLOC_MAX_CELLS cells (10 MiB,
+ * scratch is a static device array of PGE_NOALLOC_MAX_CELLS cells (4 MiB,
  * held by every GPU that loads the library until exit).  Grids with more
  * cells than that (F * NE * NE) are rejected with PGE_E_ARG, and so is any
  * grid pge_thermal rejects.  The first call on a device looks up the array's

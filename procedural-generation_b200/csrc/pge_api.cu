@@ -162,7 +162,7 @@ Layout layout(const PgeGrid &g)
     L.cubtmp_bytes = cub_temp_bytes(L.ncell, L.max_droplets);
     L.cubtmp = take(L.cubtmp_bytes);
     L.partial = take(64 * 1024);
-    L.thermal = take(40 * L.ncell);
+    L.thermal = take(24 * L.ncell);  // two fields of the thermal pass, three of the glacial one
     L.flags = take(8 * L.ncell);
     L.pwv = take(8 * L.ncell);                  // compacted values of a pairwise sum / the spawn weights' integers
     L.pwnode = take(pairwise_scratch_bytes());  // the pairwise sum's tree

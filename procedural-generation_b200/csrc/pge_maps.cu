@@ -21,8 +21,6 @@
 namespace pge {
 
 namespace {
-__constant__ int kD8[8][2] = {{1, 0}, {1, 1}, {0, 1}, {-1, 1}, {-1, 0}, {-1, -1}, {0, -1}, {1, -1}};
-
 __device__ __forceinline__ bool interior(long long c, int NE, int H, int N)
 {
     const long long r = c % ((long long)NE * NE);
@@ -326,7 +324,7 @@ void brush_spread(const PgeGrid &g, const PgeState &s, const Layout &lay, void *
 // thermal erosion (talus / creep mass wasting)
 // ---------------------------------------------------------------------------
 struct ThermalArgs {
-    int F, NE;
+    int NE;
     const double *h, *s;
     const float *metric;  // (NE,NE,3) shared or (F,NE,NE,3)
     int metric_shared;
@@ -336,120 +334,174 @@ struct ThermalArgs {
     const double *base;   // creep: submerged cells (h + s < base) are frozen
     int creep;
     double rate, cap, dep_floor;
-    double *out_total, *scale, *rscale, *new_h, *new_s;
+    double *new_h, *new_s;
 };
 
-__device__ __forceinline__ int tmask(const ThermalArgs &t, long long c)
-{
-    int m = t.mask ? t.mask[c] : PGE_MASK_ACTIVE;
-    if (t.creep && t.h[c] + t.s[c] < t.base[c]) m = PGE_MASK_FROZEN;
-    return m;
-}
+// One pass, a tile a block: the tile's surface and three cells around it in shared memory, then in turn every cell's
+// flows to its neighbours and their scale (two cells around), the share of its inflow a submerged cell has room for
+// (one cell around), and the cells' new height and sediment -- the reference's three sweeps (particle.py:1107-1227) in
+// its order of additions.  A flow and the one back share a distance, so a cell keeps four; the metric is the six faces'
+// alike, so a block takes its tile of every face in turn where the grid still fills the GPU (TH_FILL blocks).
+//
+// Bound by shared-memory reads and float64 arithmetic, not by memory.  N_c = 1024, talus and creep: 1069 us as three
+// sweeps of HBM and a copy (every neighbour's mask, surface and metric read and its distance's root taken 24 times a
+// cell); as tiles 464 with each flow computed again wherever it is used, 462 with the flows in shared memory, 406 with
+// a thread's own flows in registers and its neighbours' already at their scale.
+constexpr int TH_I = 16, TH_J = 32, TH_THREADS = TH_I * TH_J, TH_FILL = 592;
+constexpr int TH_RING = (TH_I + 4) * (TH_J + 4) - TH_THREADS;  // the two cells around the tile
+struct ThermalTile {
+    double sent[8][TH_I + 4][TH_J + 4];  // a cell's flow to each neighbour at its scale
+    double dist[4][TH_I + 4][TH_J + 4];
+    double surf[TH_I + 6][TH_J + 6];
+    double rscale[TH_I + 2][TH_J + 2];
+    uint8_t m[TH_I + 6][TH_J + 6];
+};
 
-__device__ __forceinline__ double tout(const ThermalArgs &t, long long c, int k)
+// MASKED: some cells may be frozen or outside (a mask, or the creep pass's submerged cells)
+template <bool MASKED>
+__global__ void __launch_bounds__(TH_THREADS, 2) thermal_tile_kernel(const ThermalArgs t, int faces)
 {
-    const int di = kD8[k][0], dj = kD8[k][1];
-    const long long nc = c + (long long)di * t.NE + dj;
-    const double d = (t.h[c] + t.s[c]) - (t.h[nc] + t.s[nc]);
-    if (d <= 0.0) return 0.0;
-    const long long mc = t.metric_shared ? c % ((long long)t.NE * t.NE) : c;
-    const double g0 = t.metric[3 * mc], g1 = t.metric[3 * mc + 1], g2 = t.metric[3 * mc + 2];
-    const double dist = sqrt(g0 * di * di + 2.0 * g1 * di * dj + g2 * dj * dj);
-    double talus = 0.0;
-    if (t.hard) talus = (double)__fadd_rn(t.talus_soft, __fmul_rn(t.talus_diff, t.hard[c]));
-    const double ex = d - talus * dist;
-    if (ex <= 0.0) return 0.0;
-    return 0.5 * t.rate * ex;
-}
-
-#define THERMAL_LOOP                                                                                            \
-    const long long total = (long long)t.F * t.NE * t.NE;                                                       \
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < total; c += (long long)gridDim.x * blockDim.x)
-
-__global__ void thermal_a_kernel(const ThermalArgs t)
-{
-    THERMAL_LOOP
+    extern __shared__ __align__(16) unsigned char th_smem[];
+    ThermalTile &T = *reinterpret_cast<ThermalTile *>(th_smem);
+    const int NE = t.NE, i0 = blockIdx.y * TH_I, j0 = blockIdx.x * TH_J;
+    constexpr int DI[8] = {1, 1, 0, -1, -1, -1, 0, 1}, DJ[8] = {0, 1, 1, 1, 0, -1, -1, -1};  // k + 4 is opposite k
+    const double half_rate = 0.5 * t.rate;
+    // this thread's cell of the tile, and (the first TH_RING threads) one of the cells around it
+    const int ta = threadIdx.x / TH_J, tb = threadIdx.x - ta * TH_J;
+    int ra = 0, rb = 0;
     {
-        const int i = (int)((c / t.NE) % t.NE), j = (int)(c % t.NE);
-        double ot = 0.0, sc_out = 0.0;
-        if (i >= 1 && i < t.NE - 1 && j >= 1 && j < t.NE - 1 && tmask(t, c) == PGE_MASK_ACTIVE) {
-            double S = 0.0, mx = 0.0;
-            for (int k = 0; k < 8; k++) {
-                if (tmask(t, c + (long long)kD8[k][0] * t.NE + kD8[k][1]) != PGE_MASK_ACTIVE) continue;
-                const double o = tout(t, c, k);
-                S += o;
-                if (o > mx) mx = o;
-            }
-            if (S > 0.0) {
-                double sc = 1.0;
-                if (S > 2.0 * mx) sc = 2.0 * mx / S;
-                if (t.cap > 0.0 && S * sc > t.cap) sc = t.cap / S;
-                ot = S * sc;
-                sc_out = sc;
-            }
+        const int q = threadIdx.x, w = TH_J + 4;
+        if (q < 4 * w) {  // two rows above, two below
+            const int r = q / w;
+            ra = r < 2 ? r : TH_I + r;
+            rb = q - r * w;
+        } else {  // two columns on either side
+            const int r = (q - 4 * w) / 4, c = (q - 4 * w) & 3;
+            ra = 2 + r;
+            rb = c < 2 ? c : TH_J + c;
         }
-        t.out_total[c] = ot;
-        t.scale[c] = sc_out;
     }
-}
-
-__global__ void thermal_r_kernel(const ThermalArgs t)
-{
-    THERMAL_LOOP
-    {
-        const int i = (int)((c / t.NE) % t.NE), j = (int)(c % t.NE);
-        double rs = 1.0;
-        if (i >= 1 && i < t.NE - 1 && j >= 1 && j < t.NE - 1) {
-            const double surf = t.h[c] + t.s[c];
-            if (!(surf >= 0.0 || tmask(t, c) != PGE_MASK_ACTIVE)) {
-                double inflow = 0.0;
+    auto inner = [&](int i, int j) { return i >= 1 && i < NE - 1 && j >= 1 && j < NE - 1; };
+    auto distances = [&](int a, int b, long long fb) {
+        const int i = i0 + a - 2, j = j0 + b - 2;
+        if (!inner(i, j)) return;
+        const long long mc = (t.metric_shared ? 0 : fb) + (long long)i * NE + j;
+        const double g0 = t.metric[3 * mc], g1 = t.metric[3 * mc + 1], g2 = t.metric[3 * mc + 2];
+#pragma unroll
+        for (int k = 0; k < 4; k++) T.dist[k][a][b] = sqrt(g0 * DI[k] * DI[k] + 2.0 * g1 * DI[k] * DJ[k] + g2 * DJ[k] * DJ[k]);
+    };
+    for (int f = blockIdx.z * faces; f < (int)(blockIdx.z + 1) * faces; f++) {
+        const long long fb = (long long)f * NE * NE;
+        for (int q = threadIdx.x; q < (TH_I + 6) * (TH_J + 6); q += TH_THREADS) {
+            const int a = q / (TH_J + 6), b = q - a * (TH_J + 6), i = i0 + a - 3, j = j0 + b - 3;
+            double v = 0.0;
+            int m = PGE_MASK_OUTSIDE;
+            if (i >= 0 && i < NE && j >= 0 && j < NE) {
+                const long long c = fb + (long long)i * NE + j;
+                v = t.h[c] + t.s[c];
+                m = t.mask ? t.mask[c] : PGE_MASK_ACTIVE;
+                if (t.creep && v < t.base[c]) m = PGE_MASK_FROZEN;
+            }
+            T.surf[a][b] = v;
+            if (MASKED) T.m[a][b] = (uint8_t)m;
+        }
+        if (!t.metric_shared || f == (int)blockIdx.z * faces) {
+            distances(ta + 2, tb + 2, fb);
+            if (threadIdx.x < TH_RING) distances(ra, rb, fb);
+        }
+        __syncthreads();
+        // the flows of cell (a, b) to its neighbours, their scale (0: nothing moves) and which neighbours are active
+        auto flows = [&](int a, int b, double (&o)[8], unsigned &act) {
+            const int i = i0 + a - 2, j = j0 + b - 2;
+            double sc = 0.0;
+            act = 0;
+            if (inner(i, j) && (!MASKED || T.m[a + 1][b + 1] == PGE_MASK_ACTIVE)) {
+                const double talus =
+                    t.hard ? (double)__fadd_rn(t.talus_soft, __fmul_rn(t.talus_diff, t.hard[fb + (long long)i * NE + j])) : 0.0;
+                const double surf = T.surf[a + 1][b + 1];
+                double S = 0.0, mx = 0.0;
+#pragma unroll
                 for (int k = 0; k < 8; k++) {
-                    const long long nc = c + (long long)kD8[k][0] * t.NE + kD8[k][1];
-                    const double sc = t.scale[nc];
-                    if (sc <= 0.0 || tmask(t, nc) == PGE_MASK_OUTSIDE) continue;
-                    inflow += sc * tout(t, nc, (k + 4) % 8);
+                    const double d = surf - T.surf[a + 1 + DI[k]][b + 1 + DJ[k]];
+                    const double ex = d - talus * T.dist[k & 3][a][b];
+                    o[k] = d <= 0.0 || ex <= 0.0 ? 0.0 : half_rate * ex;
+                    if (MASKED && T.m[a + 1 + DI[k]][b + 1 + DJ[k]] != PGE_MASK_ACTIVE) continue;
+                    act |= 1u << k;
+                    S += o[k];
+                    if (o[k] > mx) mx = o[k];
                 }
-                double room = -t.dep_floor - surf;
-                if (room < 0.0) room = 0.0;
-                if (inflow > room) rs = room / inflow;
+                if (S > 0.0) {
+                    sc = 1.0;
+                    if (S > 2.0 * mx) sc = 2.0 * mx / S;
+                    if (t.cap > 0.0 && S * sc > t.cap) sc = t.cap / S;
+                }
             }
+#pragma unroll
+            for (int k = 0; k < 8; k++) T.sent[k][a][b] = sc > 0.0 ? sc * o[k] : 0.0;
+            return sc;
+        };
+        double o[8];
+        unsigned act;
+        if (threadIdx.x < TH_RING) flows(ra, rb, o, act);
+        const double sc_self = flows(ta + 2, tb + 2, o, act);
+        __syncthreads();
+        // what flows into cell (a, b) (in the frame of the flows)
+        auto inflow_of = [&](int a, int b) {
+            double inflow = 0.0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) inflow += T.sent[(k + 4) & 7][a + DI[k]][b + DJ[k]];
+            return inflow;
+        };
+        for (int q = threadIdx.x; q < (TH_I + 2) * (TH_J + 2); q += TH_THREADS) {
+            const int a = q / (TH_J + 2), b = q - a * (TH_J + 2);
+            double rs = 1.0;
+            if (inner(i0 + a - 1, j0 + b - 1)) {
+                const double surf = T.surf[a + 2][b + 2];
+                if (!(surf >= 0.0 || (MASKED && T.m[a + 2][b + 2] != PGE_MASK_ACTIVE))) {
+                    const double inflow = inflow_of(a + 1, b + 1);
+                    double room = -t.dep_floor - surf;
+                    if (room < 0.0) room = 0.0;
+                    if (inflow > room) rs = room / inflow;
+                }
+            }
+            T.rscale[a][b] = rs;
         }
-        t.rscale[c] = rs;
+        __syncthreads();
+        const int i = i0 + ta, j = j0 + tb;
+        if (i < NE && j < NE) {
+            const long long c = fb + (long long)i * NE + j;
+            double h = t.h[c], s = t.s[c];
+            if (inner(i, j) && (!MASKED || T.m[ta + 3][tb + 3] == PGE_MASK_ACTIVE)) {
+                double out = 0.0;
+                if (sc_self > 0.0) {
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        if (!MASKED || (act >> k & 1u)) out += sc_self * T.rscale[ta + 1 + DI[k]][tb + 1 + DJ[k]] * o[k];
+                }
+                const double inflow = inflow_of(ta + 2, tb + 2) * T.rscale[ta + 1][tb + 1];
+                if (out > 0.0) {
+                    if (s >= out) {
+                        s -= out;
+                    } else {
+                        h -= out - s;
+                        s = 0.0;
+                    }
+                }
+                s = s + inflow;
+            }
+            t.new_h[c] = h;
+            t.new_s[c] = s;
+        }
+        __syncthreads();  // the next face's surface goes where this one's was read
     }
 }
 
-__global__ void thermal_b_kernel(const ThermalArgs t)
+template <bool MASKED>
+void thermal_launch(const ThermalArgs &t, dim3 grid, int faces, cudaStream_t st)
 {
-    THERMAL_LOOP
-    {
-        const int i = (int)((c / t.NE) % t.NE), j = (int)(c % t.NE);
-        double h = t.h[c], s = t.s[c];
-        if (i >= 1 && i < t.NE - 1 && j >= 1 && j < t.NE - 1 && tmask(t, c) == PGE_MASK_ACTIVE) {
-            double inflow = 0.0, out = 0.0;
-            const double sc_self = t.scale[c];
-            for (int k = 0; k < 8; k++) {
-                const long long nc = c + (long long)kD8[k][0] * t.NE + kD8[k][1];
-                const int mn = tmask(t, nc);
-                if (mn == PGE_MASK_OUTSIDE) continue;
-                if (sc_self > 0.0 && mn == PGE_MASK_ACTIVE) out += sc_self * t.rscale[nc] * tout(t, c, k);
-                const double sc = t.scale[nc];
-                if (sc <= 0.0) continue;
-                inflow += sc * tout(t, nc, (k + 4) % 8);
-            }
-            inflow *= t.rscale[c];
-            if (out > 0.0) {
-                if (s >= out) {
-                    s -= out;
-                } else {
-                    h -= out - s;
-                    s = 0.0;
-                }
-            }
-            s = s + inflow;
-        }
-        t.new_h[c] = h;
-        t.new_s[c] = s;
-    }
+    const int smem = (int)sizeof(ThermalTile);
+    cudaFuncSetAttribute(thermal_tile_kernel<MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    thermal_tile_kernel<MASKED><<<grid, TH_THREADS, smem, st>>>(t, faces);
 }
 
 __global__ void copy2_kernel(long long n, const double *a, const double *b, double *da, double *db)
@@ -460,51 +512,12 @@ __global__ void copy2_kernel(long long n, const double *a, const double *b, doub
     }
 }
 
-void thermal(const PgeGrid &g, PgeState &s, const Layout &lay, void *ws, double rate, double creep_rate, double cap,
-             float soft, float diff, double dep_floor, cudaStream_t st)
-{
-    double *tb = ws_ptr<double>(ws, lay.thermal);
-    const long long n = lay.ncell;
-    ThermalArgs t;
-    t.F = g.F;
-    t.NE = g.N + 2 * g.H;
-    t.h = s.height;
-    t.s = s.sediment;
-    t.metric = s.metric;
-    t.metric_shared = g.metric_shared;
-    t.talus_soft = soft;
-    t.talus_diff = diff;
-    t.mask = s.mask;
-    t.base = s.base;
-    t.dep_floor = dep_floor;
-    t.cap = cap;
-    t.out_total = tb;
-    t.scale = tb + n;
-    t.rscale = tb + 2 * n;
-    t.new_h = tb + 3 * n;
-    t.new_s = tb + 4 * n;
-    for (int pass = 0; pass < 2; pass++) {
-        if (pass == 1 && !(creep_rate > 0.0)) break;
-        t.hard = pass == 0 ? s.hardness : nullptr;
-        t.creep = pass;
-        t.rate = pass == 0 ? rate : creep_rate;
-        thermal_a_kernel<<<grid_for(n), 256, 0, st>>>(t);
-        thermal_r_kernel<<<grid_for(n), 256, 0, st>>>(t);
-        thermal_b_kernel<<<grid_for(n), 256, 0, st>>>(t);
-        copy2_kernel<<<grid_for(n), 256, 0, st>>>(n, t.new_h, t.new_s, s.height, s.sediment);
-    }
-}
-
-// the same passes on caller-provided scratch (5 * ncell doubles), for the
-// entry point that allocates nothing (pge_static.cu)
+// the talus pass from the state into the scratch (2 * n doubles) and the creep pass back into the state
 void thermal_on_scratch(const PgeGrid &g, PgeState &s, double *tb, long long n, double rate, double creep_rate, double cap,
                         float soft, float diff, double dep_floor, cudaStream_t st)
 {
     ThermalArgs t;
-    t.F = g.F;
     t.NE = g.N + 2 * g.H;
-    t.h = s.height;
-    t.s = s.sediment;
     t.metric = s.metric;
     t.metric_shared = g.metric_shared;
     t.talus_soft = soft;
@@ -513,21 +526,41 @@ void thermal_on_scratch(const PgeGrid &g, PgeState &s, double *tb, long long n, 
     t.base = s.base;
     t.dep_floor = dep_floor;
     t.cap = cap;
-    t.out_total = tb;
-    t.scale = tb + n;
-    t.rscale = tb + 2 * n;
-    t.new_h = tb + 3 * n;
-    t.new_s = tb + 4 * n;
-    for (int pass = 0; pass < 2; pass++) {
-        if (pass == 1 && !(creep_rate > 0.0)) break;
-        t.hard = pass == 0 ? s.hardness : nullptr;
-        t.creep = pass;
-        t.rate = pass == 0 ? rate : creep_rate;
-        thermal_a_kernel<<<grid_for(n), 256, 0, st>>>(t);
-        thermal_r_kernel<<<grid_for(n), 256, 0, st>>>(t);
-        thermal_b_kernel<<<grid_for(n), 256, 0, st>>>(t);
-        copy2_kernel<<<grid_for(n), 256, 0, st>>>(n, t.new_h, t.new_s, s.height, s.sediment);
+    t.h = s.height;
+    t.s = s.sediment;
+    t.hard = s.hardness;
+    t.creep = 0;
+    t.rate = rate;
+    t.new_h = tb;
+    t.new_s = tb + n;
+    dim3 grid((t.NE + TH_J - 1) / TH_J, (t.NE + TH_I - 1) / TH_I, g.F);
+    int faces = 1;
+    if (grid.x * grid.y >= TH_FILL) {
+        faces = g.F;
+        grid.z = 1;
     }
+    if (t.mask)
+        thermal_launch<true>(t, grid, faces, st);
+    else
+        thermal_launch<false>(t, grid, faces, st);
+    if (!(creep_rate > 0.0)) {
+        copy2_kernel<<<grid_for(n), 256, 0, st>>>(n, tb, tb + n, s.height, s.sediment);
+        return;
+    }
+    t.h = tb;
+    t.s = tb + n;
+    t.hard = nullptr;
+    t.creep = 1;
+    t.rate = creep_rate;
+    t.new_h = s.height;
+    t.new_s = s.sediment;
+    thermal_launch<true>(t, grid, faces, st);
+}
+
+void thermal(const PgeGrid &g, PgeState &s, const Layout &lay, void *ws, double rate, double creep_rate, double cap, float soft,
+             float diff, double dep_floor, cudaStream_t st)
+{
+    thermal_on_scratch(g, s, ws_ptr<double>(ws, lay.thermal), lay.ncell, rate, creep_rate, cap, soft, diff, dep_floor, st);
 }
 
 struct UpliftValue {

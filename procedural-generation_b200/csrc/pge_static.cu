@@ -4,9 +4,9 @@
 // allocate device memory at all: a host application that owns the whole
 // device heap through its own pool and forbids any other allocation, or a
 // loop that must not pay cudaMalloc's latency and implicit device
-// synchronisation.  pge_thermal_noalloc serves them: its scratch (five
+// synchronisation.  pge_thermal_noalloc serves them: its scratch (two
 // float64 values per cell) is a file-scope __device__ array of fixed size,
-// PGE_NOALLOC_MAX_CELLS cells (10 MiB), which every GPU that loads the
+// PGE_NOALLOC_MAX_CELLS cells (4 MiB), which every GPU that loads the
 // library holds until the process exits.
 //
 // Host code cannot pass that array's name to a kernel: in host code the
@@ -31,7 +31,7 @@
 namespace pge {
 namespace {
 
-__device__ __align__(256) double g_thermal_scratch[5 * (size_t)PGE_NOALLOC_MAX_CELLS];
+__device__ __align__(256) double g_thermal_scratch[2 * (size_t)PGE_NOALLOC_MAX_CELLS];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
