@@ -23,8 +23,8 @@ namespace pge {
 namespace {
 __device__ __forceinline__ bool interior(long long c, int NE, int H, int N)
 {
-    const long long r = c % ((long long)NE * NE);
-    const int i = (int)(r / NE), j = (int)(r % NE);
+    const unsigned u = (unsigned)c, row = u / (unsigned)NE;  // (a cell index fits 31 bits)
+    const int j = (int)(u - row * (unsigned)NE), i = (int)(row % (unsigned)NE);
     return i >= H && i < H + N && j >= H && j < H + N;
 }
 
@@ -596,21 +596,15 @@ struct Positive {
 // one; a longer range is split at n2 = n/2 rounded down to a multiple of 8 and
 // the two halves' sums added.  (numpy's pairwise_sum, the reduction loop of
 // np.add; checked against np.sum on ranges of 1..5000 values of mixed
-// magnitudes.)  The top of the tree is expanded breadth-first into at most
-// PW_MAX_LEVEL_NODES nodes a level (one block, a level at a time); the bottom
-// nodes are summed one per thread and the tree is folded back up in order (one
-// block, a level at a time).
+// magnitudes.)  The split depends on the count alone, so a node finds its own
+// range by walking down from the root: nothing is planned or stored.  Eight
+// lanes sum a leaf, a block folds its PW_BLOCK_NODES consecutive nodes, and one
+// block folds the blocks.
 // ---------------------------------------------------------------------------
 constexpr int PW_LEAF = 128;
-constexpr int PW_MAX_LEVELS = 24;
-constexpr int PW_MAX_LEVEL_NODES = 32768;
+constexpr int PW_MAX_DEPTH = 20;  // nodes at most 2^20: a longer array's leaves are summed by one lane each
+constexpr int PW_BLOCK_LOG = 7, PW_BLOCK_NODES = 1 << PW_BLOCK_LOG;
 constexpr int PW_THREADS = 1024;
-
-struct PwNode {
-    long long lo, n;
-    int child, nchild;  // children in the next level
-    double sum;
-};
 
 __device__ double pw_leaf(const double *a, long long n)
 {
@@ -680,104 +674,94 @@ __device__ double pw_sum(const double *a, long long n)
     }
 }
 
-// one block of PW_THREADS: a level's nodes split among the threads in order, each thread's children placed
-// after those of the threads before it (a block scan of the counts)
-__global__ void __launch_bounds__(PW_THREADS) pw_plan_kernel(const long long *count, PwNode *nodes, int *level_start)
+// a node's sum, or that it lies below a leaf (there is nothing in it: the leaf stands at its first descendant)
+struct PwSum {
+    double sum;
+    int there;
+};
+__device__ __forceinline__ PwSum pw_add(const PwSum &l, const PwSum &r) { return r.there ? PwSum{l.sum + r.sum, 1} : l; }
+
+__global__ void __launch_bounds__(256) pw_leaf_kernel(const double *a, const long long *count, int depth, PwSum *part)
 {
-    typedef cub::BlockScan<int, PW_THREADS> Scan;
-    typedef cub::BlockReduce<long long, PW_THREADS> Reduce;
-    __shared__ typename Scan::TempStorage scan_tmp;
-    __shared__ typename Reduce::TempStorage red_tmp;
-    __shared__ long long s_biggest;
-    __shared__ int s_next;
-    const int t = threadIdx.x;
+    __shared__ PwSum node[PW_BLOCK_NODES];
+    const int lane8 = threadIdx.x & 7, group = threadIdx.x >> 3;
+    const unsigned eight = 0xffu << (threadIdx.x & 24);
     const long long M = *count;
-    if (t == 0) {
-        nodes[0] = PwNode{0, M, -1, 0, 0.0};
-        level_start[0] = 0;
+    for (int t = group; t < PW_BLOCK_NODES; t += 32) {
+        const unsigned k = blockIdx.x * PW_BLOCK_NODES + t;
+        long long lo = 0, n = M;
+        bool there = k < 1u << depth;
+        for (int l = depth - 1; l >= 0 && there; l--) {
+            const unsigned right = k >> l & 1u;
+            if (n <= PW_LEAF) {  // a leaf above: it stands at its first descendant
+                there = (k & ((1u << (l + 1)) - 1u)) == 0;
+                break;
+            }
+            const long long n2 = pw_split(n);
+            lo += right ? n2 : 0;
+            n = right ? n - n2 : n2;
+        }
+        double sum = 0.0;
+        if (there && n > PW_LEAF) {
+            if (lane8 == 0) sum = pw_sum(a + lo, n);
+        } else if (there && n < 8) {
+            if (lane8 == 0) sum = pw_leaf(a + lo, n);
+        } else if (there) {
+            const double *p = a + lo;
+            const int m = (int)n - (int)n % 8;
+            double r = p[lane8];
+            for (int i = 8; i < m; i += 8) r += p[i + lane8];
+            r += __shfl_xor_sync(eight, r, 1);  // (commutative: every lane has r0 + r1, then (r0 + r1) + (r2 + r3), ..)
+            r += __shfl_xor_sync(eight, r, 2);
+            r += __shfl_xor_sync(eight, r, 4);
+            for (int i = m; i < (int)n; i++) r += p[i];
+            sum = r;
+        }
+        if (lane8 == 0) node[t] = PwSum{sum, there};
     }
     __syncthreads();
-    int nl = 0, begin = 0, end = 1;
-    while (nl + 1 < PW_MAX_LEVELS) {
-        const int nnodes = end - begin;
-        const int per = (nnodes + PW_THREADS - 1) / PW_THREADS;
-        const int k0 = begin + t * per, k1 = min(k0 + per, end);
-        long long big = 0;
-        int nch = 0;
-        for (int k = k0; k < k1; k++) {
-            big = nodes[k].n > big ? nodes[k].n : big;
-            nch += nodes[k].n > PW_LEAF ? 2 : 1;
-        }
-        const long long b = Reduce(red_tmp).Reduce(big, cub::Max());
-        if (t == 0) s_biggest = b;
+    for (int w = PW_BLOCK_NODES / 2; w > 0; w >>= 1) {
+        PwSum s;
+        if ((int)threadIdx.x < w) s = pw_add(node[2 * threadIdx.x], node[2 * threadIdx.x + 1]);
         __syncthreads();
-        if (s_biggest <= 8 * PW_LEAF || 2 * nnodes > PW_MAX_LEVEL_NODES) break;
-        int off, total;
-        Scan(scan_tmp).ExclusiveSum(nch, off, total);
-        int next = end + off;
-        for (int k = k0; k < k1; k++) {
-            PwNode &nd = nodes[k];
-            nd.child = next;
-            if (nd.n > PW_LEAF) {
-                const long long n2 = pw_split(nd.n);
-                nodes[next++] = PwNode{nd.lo, n2, -1, 0, 0.0};
-                nodes[next++] = PwNode{nd.lo + n2, nd.n - n2, -1, 0, 0.0};
-                nd.nchild = 2;
-            } else {
-                nodes[next++] = PwNode{nd.lo, nd.n, -1, 0, 0.0};  // a leaf passes down unchanged
-                nd.nchild = 1;
-            }
-        }
-        if (t == 0) s_next = end + total;
-        __syncthreads();
-        begin = end;
-        end = s_next;
-        nl++;
-        if (t == 0) level_start[nl] = begin;
+        if ((int)threadIdx.x < w) node[threadIdx.x] = s;
         __syncthreads();
     }
-    if (t == 0) {
-        level_start[nl + 1] = end;
-        level_start[PW_MAX_LEVELS + 1] = nl;  // the bottom level's index
-    }
+    if (threadIdx.x == 0) part[blockIdx.x] = node[0];
 }
 
-__global__ void pw_bottom_kernel(const double *a, PwNode *nodes, const int *level_start)
+// folds the blocks' sums (a power of two of them); out = the sum, or with mean_out the sum / count
+__global__ void __launch_bounds__(PW_THREADS) pw_fold_kernel(PwSum *part, int n, const long long *count, double *out, int mean_out)
 {
-    const int nl = level_start[PW_MAX_LEVELS + 1];
-    const int begin = level_start[nl], end = level_start[nl + 1];
-    for (int k = begin + blockIdx.x * blockDim.x + threadIdx.x; k < end; k += gridDim.x * blockDim.x)
-        nodes[k].sum = pw_sum(a + nodes[k].lo, nodes[k].n);
-}
-
-// folds the levels back up, a level at a time (one block); out = the sum, or with mean_out the sum / count
-__global__ void __launch_bounds__(PW_THREADS) pw_fold_kernel(PwNode *nodes, const int *level_start, const long long *count,
-                                                             double *out, int mean_out)
-{
-    const int nl = level_start[PW_MAX_LEVELS + 1];
-    for (int l = nl - 1; l >= 0; l--) {
-        for (int k = level_start[l] + threadIdx.x; k < level_start[l + 1]; k += blockDim.x) {
-            PwNode &nd = nodes[k];
-            nd.sum = nd.nchild == 2 ? nodes[nd.child].sum + nodes[nd.child + 1].sum : nodes[nd.child].sum;
+    for (int w = n / 2; w > 0; w >>= 1) {
+        // (each round reads the places 2k, 2k + 1 and writes the place k: the rounds of one width go in order)
+        for (int k0 = 0; k0 < w; k0 += blockDim.x) {
+            const int k = k0 + threadIdx.x;
+            PwSum s{0.0, 0};
+            if (k < w) s = pw_add(part[2 * k], part[2 * k + 1]);
+            __syncthreads();
+            if (k < w) part[k] = s;
+            __syncthreads();
         }
-        __syncthreads();
     }
     if (threadIdx.x == 0) {
         const long long M = *count;
-        *out = mean_out ? (M > 0 ? nodes[0].sum / (double)M : 0.0) : nodes[0].sum;
+        *out = mean_out ? (M > 0 ? part[0].sum / (double)M : 0.0) : part[0].sum;
     }
 }
 
-size_t pairwise_scratch_bytes() { return sizeof(PwNode) * (size_t)PW_MAX_LEVELS * PW_MAX_LEVEL_NODES + 256; }
+size_t pairwise_scratch_bytes() { return sizeof(PwSum) << (PW_MAX_DEPTH - PW_BLOCK_LOG); }
 
-// sum (or mean) of a[0, *count) in numpy's pairwise order, written to *out on the stream
-void pairwise_sum(const double *a, const long long *count, void *scratch, double *out, int mean, cudaStream_t st)
+// sum (or mean) of a[0, *count), at most n_max values, in numpy's pairwise order, written to *out on the stream
+void pairwise_sum(const double *a, const long long *count, long long n_max, void *scratch, double *out, int mean, cudaStream_t st)
 {
-    PwNode *nodes = static_cast<PwNode *>(scratch);
-    int *level_start = reinterpret_cast<int *>(nodes + (size_t)PW_MAX_LEVELS * PW_MAX_LEVEL_NODES);
-    pw_plan_kernel<<<1, PW_THREADS, 0, st>>>(count, nodes, level_start);
-    pw_bottom_kernel<<<(PW_MAX_LEVEL_NODES + 127) / 128, 128, 0, st>>>(a, nodes, level_start);
-    pw_fold_kernel<<<1, PW_THREADS, 0, st>>>(nodes, level_start, count, out, mean);
+    PwSum *part = static_cast<PwSum *>(scratch);
+    // a range at depth l is at most n / 2^l + 16 long: deep enough that every node fits a leaf
+    int depth = PW_BLOCK_LOG;
+    while (depth < PW_MAX_DEPTH && (n_max >> depth) > PW_LEAF - 32) depth++;
+    const int blocks = 1 << (depth - PW_BLOCK_LOG);
+    pw_leaf_kernel<<<blocks, 256, 0, st>>>(a, count, depth, part);
+    pw_fold_kernel<<<1, PW_THREADS, 0, st>>>(part, blocks, count, out, mean);
 }
 
 // ---------------------------------------------------------------------------
@@ -814,14 +798,14 @@ void uplift(const PgeGrid &g, PgeState &s, const Layout &lay, void *ws, double c
                                    thrust::make_transform_iterator(c0, UpliftValue{s.uplift, cap, use_cap}),
                                    thrust::make_transform_iterator(c0, InteriorActive{NE, g.H, g.N, s.mask}), vals, pcount,
                                    (int)lay.ncell, st);
-        pairwise_sum(vals, pcount, ws_ptr<void>(ws, lay.pwnode), mean, 1, st);
+        pairwise_sum(vals, pcount, lay.ncell, ws_ptr<void>(ws, lay.pwnode), mean, 1, st);
     }
     uplift_add_kernel<<<grid_for(lay.ncell), 256, 0, st>>>(lay.ncell, s.height, s.uplift, s.mask, cap, use_cap,
                                                            g.spherical ? mean : nullptr, scale);
 }
 
 // ---------------------------------------------------------------------------
-// datum: k-th smallest interior surface by an 8-pass radix select on the
+// datum: k-th smallest interior surface by a 6-pass radix select on the
 // order-preserving 64-bit image of the float64 keys
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long okey(double v)
@@ -836,54 +820,77 @@ __device__ __forceinline__ double unokey(unsigned long long k)
     return __longlong_as_double((long long)b);
 }
 
+// digits of 11 bits, the last of 9: six passes
+constexpr int SEL_BITS = 11, SEL_BINS = 1 << SEL_BITS, SEL_THREADS = 512;
 struct SelectState {
     unsigned long long prefix;  // digits found so far (high bits)
     long long k;                // rank still sought inside the prefix
-    unsigned int hist[256];
+    unsigned int done;          // blocks that have added their histogram
+    unsigned int hist[SEL_BINS];
 };
 
-__global__ void select_hist_kernel(long long ncell, int NE, int H, int N, const double *h, const double *s, SelectState *ss,
-                                   int shift)
+// one digit: every block adds its histogram of the keys inside the prefix, the last one finds the digit of the rank
+// sought and clears the histogram for the next
+__global__ void __launch_bounds__(SEL_THREADS) select_digit_kernel(long long ncell, int NE, int H, int N, const double *__restrict__ h,
+                                                                   const double *__restrict__ s, SelectState *ss, int shift, int bits)
 {
-    __shared__ unsigned int sh[256];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) sh[i] = 0;
+    __shared__ unsigned int sh[SEL_BINS];
+    __shared__ bool last;
+    for (int i = threadIdx.x; i < SEL_BINS; i += SEL_THREADS) sh[i] = 0;
     __syncthreads();
     const unsigned long long prefix = ss->prefix;
-    const unsigned long long hmask = shift >= 56 ? 0ull : (~0ull << (shift + 8));
+    const unsigned long long hmask = shift + bits >= 64 ? 0ull : (~0ull << (shift + bits));
+    const unsigned digit = (1u << bits) - 1u;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncell; c += (long long)gridDim.x * blockDim.x) {
         if (!interior(c, NE, H, N)) continue;
         const unsigned long long k = okey(h[c] + s[c]);
         if ((k & hmask) != (prefix & hmask)) continue;
-        atomicAdd(&sh[(k >> shift) & 255], 1u);
+        atomicAdd(&sh[(unsigned)(k >> shift) & digit], 1u);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 256; i += blockDim.x)
+    for (int i = threadIdx.x; i < SEL_BINS; i += SEL_THREADS)
         if (sh[i]) atomicAdd(&ss->hist[i], sh[i]);
-}
-
-__global__ void select_pick_kernel(SelectState *ss, int shift)
-{
-    if (threadIdx.x == 0) {
-        long long k = ss->k;
-        int d = 0;
-        for (; d < 255; d++) {
-            const long long c = ss->hist[d];
-            if (k < c) break;
-            k -= c;
-        }
-        ss->k = k;
-        ss->prefix |= (unsigned long long)d << shift;
-    }
+    __threadfence();
     __syncthreads();
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) ss->hist[i] = 0;
+    if (threadIdx.x == 0) last = atomicAdd(&ss->done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // the digit: the first bin whose running count passes the rank
+    typedef cub::BlockScan<long long, SEL_THREADS> Scan;
+    __shared__ typename Scan::TempStorage tmp;
+    constexpr int PER = SEL_BINS / SEL_THREADS;
+    unsigned int n[PER];
+    long long mine = 0;
+    for (int q = 0; q < PER; q++) {
+        n[q] = ((volatile unsigned int *)ss->hist)[threadIdx.x * PER + q];
+        mine += n[q];
+    }
+    long long before;
+    Scan(tmp).ExclusiveSum(mine, before);
+    const long long k = ss->k;
+    __syncthreads();  // every thread has read the rank
+    long long at = before;
+    for (int q = 0; q < PER; q++) {
+        const int bin = threadIdx.x * PER + q;
+        // (a rank beyond the keys takes the last digit)
+        if ((k >= at && k < at + (long long)n[q]) || (bin == (int)digit && k >= at + (long long)n[q])) {
+            ss->k = k - at;
+            ss->prefix = prefix | (unsigned long long)bin << shift;
+        }
+        at += n[q];
+        ss->hist[bin] = 0;
+    }
+    if (threadIdx.x == 0) ss->done = 0;
 }
 
 __global__ void select_init_kernel(SelectState *ss, long long k)
 {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) ss->hist[i] = 0;
+    for (int i = threadIdx.x; i < SEL_BINS; i += blockDim.x) ss->hist[i] = 0;
     if (threadIdx.x == 0) {
         ss->prefix = 0;
         ss->k = k;
+        ss->done = 0;
     }
 }
 
@@ -919,9 +926,11 @@ void hold_datum(const PgeGrid &g, PgeState &s, const Layout &lay, void *ws, doub
     }
     SelectState *ss = ws_ptr<SelectState>(ws, lay.partial + 4 * RED_BLOCKS * sizeof(double));
     select_init_kernel<<<1, 256, 0, st>>>(ss, k);
-    for (int shift = 56; shift >= 0; shift -= 8) {
-        select_hist_kernel<<<grid_reduce(lay.ncell), 256, 0, st>>>(lay.ncell, NE, g.H, g.N, s.height, s.sediment, ss, shift);
-        select_pick_kernel<<<1, 256, 0, st>>>(ss, shift);
+    for (int top = 64; top > 0;) {
+        const int bits = top < SEL_BITS ? top : SEL_BITS;
+        top -= bits;
+        select_digit_kernel<<<grid_reduce(lay.ncell, SEL_THREADS), SEL_THREADS, 0, st>>>(lay.ncell, NE, g.H, g.N, s.height, s.sediment, ss,
+                                                                                         top, bits);
     }
     datum_shift_kernel<<<grid_for(lay.ncell), 256, 0, st>>>(lay.ncell, s.height, s.base, ss, level, plus_one, shift_dev);
 }
@@ -1166,7 +1175,7 @@ cudaError_t spawn_rain(const PgeGrid &g, const PgeState &s, const Layout &lay, v
     tb = lay.cubtmp_bytes;
     e = cub::DeviceSelect::If(ws_ptr<void>(ws, lay.cubtmp), tb, w, wc, nsel, (int)lay.ncell, Positive{}, st);
     if (e != cudaSuccess) return e;
-    if (total_dev) pairwise_sum(wc, nsel, ws_ptr<void>(ws, lay.pwnode), total_dev, 0, st);
+    if (total_dev) pairwise_sum(wc, nsel, lay.ncell, ws_ptr<void>(ws, lay.pwnode), total_dev, 0, st);
     tb = lay.cubtmp_bytes;
     e = cub::DeviceRadixSort::SortKeys(ws_ptr<void>(ws, lay.cubtmp), tb, u, keys, (int)P, 0, 64, st);
     if (e != cudaSuccess) return e;
@@ -1244,46 +1253,78 @@ void slope_erode_cap(const PgeGrid &g, const PgeState &s, double k, double exit_
 //                                                  Laplacian in cell units, for the step bound)
 // float64 in the reference's operation order (no FMA in this file)
 // ---------------------------------------------------------------------------
-__global__ void smooth_step_kernel(int F, int NE, const double *__restrict__ d, const float *__restrict__ ginv_f,
-                                   const float *__restrict__ sq_f, double c2, double kappa, int keep, double *__restrict__ out)
+// A thread takes SM_ROWS cells of its column on SM_FACES faces: the metric is the same on every face, so the edges'
+// coefficients (four means of strided float32 tables, half the reads) are made once for all of them.  Bound by the
+// latency of its loads at the occupancy its registers leave (ncu: float64 pipe 34 %, L1 30 %).  N_c = 725, one step:
+// a cell a thread 46.4 us; rows x faces 1 x 1 43, 1 x 3 33, 1 x 6 29.0, 2 x 6 34, 4 x 2 59; the next face's cells read
+// ahead 29.3.
+constexpr int SM_X = 32, SM_Y = 8, SM_ROWS = 1, SM_FACES = 6;
+struct SmoothEdge {
+    double sv, g, x;  // mean sqrt(g), mean metric across the edge, half the mean mixed metric
+};
+__global__ void __launch_bounds__(SM_X *SM_Y) smooth_step_kernel(int F, int NE, const double *__restrict__ d, const float *__restrict__ ginv,
+                                                                 const float *__restrict__ sq, double c2, double kappa, int keep,
+                                                                 double *__restrict__ out)
 {
-    const long long n = (long long)F * NE * NE;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        const long long r = c % ((long long)NE * NE);
-        const int i = (int)(r / NE), j = (int)(r - (long long)i * NE);
-        double lap64 = 0.0;
-        if (i >= 1 && i <= NE - 2 && j >= 1 && j <= NE - 2) {
-            // the metric tables are the same on every face: index them by (i, j)
-            auto G = [&](int ii, int jj, int k) { return (double)ginv_f[((long long)ii * NE + jj) * 3 + k]; };
-            auto S = [&](int ii, int jj) { return (double)sq_f[(long long)ii * NE + jj]; };
-            auto D = [&](int ii, int jj) { return d[c + (long long)(ii - i) * NE + (jj - j)]; };
-            const double fj_c = 0.5 * (D(i, j + 1) - D(i, j - 1));
-            const double fj_p = 0.5 * (D(i + 1, j + 1) - D(i + 1, j - 1));
-            const double fj_m = 0.5 * (D(i - 1, j + 1) - D(i - 1, j - 1));
-            const double fi_c = 0.5 * (D(i + 1, j) - D(i - 1, j));
-            const double fi_p = 0.5 * (D(i + 1, j + 1) - D(i - 1, j + 1));
-            const double fi_m = 0.5 * (D(i + 1, j - 1) - D(i - 1, j - 1));
-            double gii = 0.5 * (G(i, j, 0) + G(i + 1, j, 0));
-            double gij = 0.5 * (G(i, j, 1) + G(i + 1, j, 1));
-            double sv = 0.5 * (S(i, j) + S(i + 1, j));
-            const double Fi_p = sv * (gii * (D(i + 1, j) - D(i, j)) + gij * 0.5 * (fj_c + fj_p));
-            gii = 0.5 * (G(i, j, 0) + G(i - 1, j, 0));
-            gij = 0.5 * (G(i, j, 1) + G(i - 1, j, 1));
-            sv = 0.5 * (S(i, j) + S(i - 1, j));
-            const double Fi_m = sv * (gii * (D(i, j) - D(i - 1, j)) + gij * 0.5 * (fj_c + fj_m));
-            double gjj = 0.5 * (G(i, j, 2) + G(i, j + 1, 2));
-            gij = 0.5 * (G(i, j, 1) + G(i, j + 1, 1));
-            sv = 0.5 * (S(i, j) + S(i, j + 1));
-            const double Fj_p = sv * (gjj * (D(i, j + 1) - D(i, j)) + gij * 0.5 * (fi_c + fi_p));
-            gjj = 0.5 * (G(i, j, 2) + G(i, j - 1, 2));
-            gij = 0.5 * (G(i, j, 1) + G(i, j - 1, 1));
-            sv = 0.5 * (S(i, j) + S(i, j - 1));
-            const double Fj_m = sv * (gjj * (D(i, j) - D(i, j - 1)) + gij * 0.5 * (fi_c + fi_m));
-            const double lap = (Fi_p - Fi_m + Fj_p - Fj_m) / S(i, j);
-            lap64 = (double)(float)(lap / c2);  // per m^2, a float32 field
+    const int j = blockIdx.x * SM_X + threadIdx.x, i0 = (blockIdx.y * SM_Y + threadIdx.y) * SM_ROWS;
+    if (j >= NE || i0 >= NE) return;
+    const int f0 = blockIdx.z * SM_FACES;
+    const long long plane = (long long)NE * NE;
+    const bool inner_j = j >= 1 && j <= NE - 2;
+    SmoothEdge ei[SM_ROWS + 1], ep[SM_ROWS], em[SM_ROWS];  // to the row above each row (and below the last), to j + 1, to j - 1
+    double s_c[SM_ROWS];
+    if (inner_j) {
+        auto edge = [&](int a, int b, int k) {  // between the cells at flat places a and b, along axis k / 2
+            return SmoothEdge{0.5 * ((double)sq[a] + (double)sq[b]), 0.5 * ((double)ginv[3 * a + k] + (double)ginv[3 * b + k]),
+                              0.5 * ((double)ginv[3 * a + 1] + (double)ginv[3 * b + 1]) * 0.5};
+        };
+#pragma unroll
+        for (int r = 0; r <= SM_ROWS; r++) {
+            const int i = i0 + r, at = i * NE + j;
+            if (i >= 1 && i <= NE - 1) ei[r] = edge(at, at - NE, 0);
+            if (r < SM_ROWS && i >= 1 && i <= NE - 2) {
+                s_c[r] = (double)sq[at];
+                ep[r] = edge(at, at + 1, 2);
+                em[r] = edge(at, at - 1, 2);
+            }
         }
-        const double upd = kappa * lap64 * c2;
-        out[c] = keep ? d[c] + upd : upd;
+    }
+#pragma unroll
+    for (int q = 0; q < SM_FACES; q++) {
+        if (f0 + q >= F) break;
+        const double *df = d + (f0 + q) * plane;
+        double *of = out + (f0 + q) * plane;
+        double v[SM_ROWS + 2][3];
+#pragma unroll
+        for (int r = 0; r < SM_ROWS + 2; r++) {
+            const int i = i0 + r - 1;
+            const bool in = i >= 0 && i < NE;
+            const double *p = df + (long long)i * NE + j;
+            v[r][0] = in && inner_j ? p[-1] : 0.0;
+            v[r][1] = in ? p[0] : 0.0;
+            v[r][2] = in && inner_j ? p[1] : 0.0;
+        }
+        // the flux between rows r - 1 and r of v
+        auto flux_i = [&](const SmoothEdge &e, int r) {
+            const double fl = 0.5 * (v[r - 1][2] - v[r - 1][0]), fh = 0.5 * (v[r][2] - v[r][0]);
+            return e.sv * (e.g * (v[r][1] - v[r - 1][1]) + e.x * (fl + fh));
+        };
+#pragma unroll
+        for (int r = 0; r < SM_ROWS; r++) {
+            const int i = i0 + r;
+            if (i >= NE) break;
+            double lap64 = 0.0;  // (0 on the outer ring)
+            if (inner_j && i >= 1 && i <= NE - 2) {
+                const double Fi_m = flux_i(ei[r], r + 1), Fi_p = flux_i(ei[r + 1], r + 2);
+                const double fi_m = 0.5 * (v[r + 2][0] - v[r][0]), fi_c = 0.5 * (v[r + 2][1] - v[r][1]), fi_p = 0.5 * (v[r + 2][2] - v[r][2]);
+                const double Fj_p = ep[r].sv * (ep[r].g * (v[r + 1][2] - v[r + 1][1]) + ep[r].x * (fi_c + fi_p));
+                const double Fj_m = em[r].sv * (em[r].g * (v[r + 1][1] - v[r + 1][0]) + em[r].x * (fi_c + fi_m));
+                const double lap = (Fi_p - Fi_m + Fj_p - Fj_m) / s_c[r];
+                lap64 = (double)(float)(lap / c2);  // per m^2, a float32 field
+            }
+            const double upd = kappa * lap64 * c2;
+            of[(long long)i * NE + j] = keep ? v[r + 1][1] + upd : upd;
+        }
     }
 }
 
@@ -1292,7 +1333,8 @@ void smooth_step(const PgeGrid &g, const double *in, const float *metric_inv, co
 {
     const int NE = g.N + 2 * g.H;
     const double c2 = cell_m * cell_m;
-    smooth_step_kernel<<<grid_for((long long)g.F * NE * NE), 256, 0, st>>>(g.F, NE, in, metric_inv, sqrt_det, c2, kappa, keep, out);
+    const dim3 grid((NE + SM_X - 1) / SM_X, (NE + SM_Y * SM_ROWS - 1) / (SM_Y * SM_ROWS), (g.F + SM_FACES - 1) / SM_FACES);
+    smooth_step_kernel<<<grid, dim3(SM_X, SM_Y), 0, st>>>(g.F, NE, in, metric_inv, sqrt_det, c2, kappa, keep, out);
 }
 
 }  // namespace pge

@@ -22,9 +22,9 @@ size_t cub_temp_bytes(int64_t ncell, int64_t max_droplets);
 // the erode / deposit brush (PgeParams.brush_radius): the net change the wave apply accumulated since the last call,
 // spread over each cell's footprint in integer shares, added to the accumulators' net-change column
 void brush_spread(const PgeGrid &g, const PgeState &s, const Layout &lay, void *ws, int r, cudaStream_t st);
-// numpy's pairwise float64 sum (mean = 1: divided by the count) of a[0, *count), on the stream
+// numpy's pairwise float64 sum (mean = 1: divided by the count) of a[0, *count), *count <= n_max, on the stream
 size_t pairwise_scratch_bytes();
-void pairwise_sum(const double *a, const long long *count, void *scratch, double *out, int mean, cudaStream_t st);
+void pairwise_sum(const double *a, const long long *count, long long n_max, void *scratch, double *out, int mean, cudaStream_t st);
 // the planet's lake balance on the host (pge_lakes.cpp), with erosion.lake_fill's settle when fill is set; 0,
 // -1 when a land cell has no flow direction, -2 when more lakes take load than fill->lake_room_cap
 int lake_balance_host(int N, int H, const int32_t *owner, const float *metric, const float *cell_area, double cell_size_m,
