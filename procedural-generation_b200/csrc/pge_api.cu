@@ -183,10 +183,7 @@ Layout layout(const PgeGrid &g)
     L.w_keys1 = take(8 * ws);
     L.w_vals0 = take(4 * ws);
     L.w_vals1 = take(4 * ws);
-    L.w_runstart = take(4 * ws);
-    L.w_segpos = take(4 * ws);
-    L.w_runscan = take(4 * ws);
-    L.w_segscan = take(4 * ws);
+    for (size_t &x : L.w_fin) x = take(4 * ws);
     L.w_temp_bytes = ordered_temp_bytes(ws, L.max_wave);
     L.w_temp = take(L.w_temp_bytes);
     L.w_dth = take(4 * L.max_wave);
@@ -357,11 +354,11 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
                 pw.lakes = s->lakes;
                 pw.lake_load = s->lake_load;
                 pw.rest = ws_ptr<double>(ws, lay.w_park_rest);
-                // the cell sort's scan buffers are free until the wave's own ranks
-                pw.keys_in = ws_ptr<uint32_t>(ws, lay.w_runstart);
-                pw.keys_out = ws_ptr<uint32_t>(ws, lay.w_segpos);
-                pw.vals_in = ws_ptr<int32_t>(ws, lay.w_runscan);
-                pw.vals_out = ws_ptr<int32_t>(ws, lay.w_segscan);
+                // the finish's rows are free until the wave's own finish, the cell sort's values until its ranks
+                pw.keys_in = ws_ptr<uint32_t>(ws, lay.w_fin[0]);
+                pw.keys_out = ws_ptr<uint32_t>(ws, lay.w_fin[1]);
+                pw.vals_in = ws_ptr<int32_t>(ws, lay.w_fin[2]);
+                pw.vals_out = ws_ptr<int32_t>(ws, lay.w_vals0);
                 pw.temp = ws_ptr<void>(ws, lay.w_temp);
                 pw.temp_bytes = lay.w_temp_bytes;
             }
@@ -371,14 +368,11 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
             while ((1LL << cbits) < lay.ncell + 1) cbits++;
             ow.end_bit = cbits;
             ow.invalid = (1ull << cbits) - 1ull;
-            ow.keys_in = ws_ptr<unsigned long long>(ws, lay.w_keys0);
-            ow.keys_out = ws_ptr<unsigned long long>(ws, lay.w_keys1);
+            ow.keys_in = ws_ptr<SortKey>(ws, lay.w_keys0);
+            ow.keys_out = ws_ptr<SortKey>(ws, lay.w_keys1);
             ow.vals_in = ws_ptr<int32_t>(ws, lay.w_vals0);
             ow.vals_out = ws_ptr<int32_t>(ws, lay.w_vals1);
-            ow.runstart = ws_ptr<int32_t>(ws, lay.w_runstart);
-            ow.segpos = ws_ptr<int32_t>(ws, lay.w_segpos);
-            ow.runscan = ws_ptr<int32_t>(ws, lay.w_runscan);
-            ow.segscan = ws_ptr<int32_t>(ws, lay.w_segscan);
+            for (int k = 0; k < 3; k++) ow.fin[k] = ws_ptr<float>(ws, lay.w_fin[k]);
             ow.temp = ws_ptr<void>(ws, lay.w_temp);
             ow.temp_bytes = lay.w_temp_bytes;
             ow.offsets = lay.cap >= COMPACT_CAP ? ws_ptr<long long>(ws, lay.w_offsets) : nullptr;

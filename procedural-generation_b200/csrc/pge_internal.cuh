@@ -62,10 +62,11 @@ struct Layout {
     size_t cellA, cellB, live, metric8, route2, acc4, pend, tkey, town, counters, sortkeys, sortvals, cdf, cubtmp, cubtmp_bytes,
         partial, thermal, flags, pwv, pwnode, spread, total;
     // ordered apply (exact mode): one wave's change lists and ranks
-    size_t w_cell, w_delta, w_vol, w_mom, w_count, w_death, w_rec, w_keys0, w_keys1, w_vals0, w_vals1, w_runstart,
-        w_segpos, w_runscan, w_segscan, w_temp, w_temp_bytes, w_dth, w_keep, hand, terr, error;
+    size_t w_cell, w_delta, w_vol, w_mom, w_count, w_death, w_rec, w_keys0, w_keys1, w_vals0,
+        w_vals1, w_temp, w_temp_bytes, w_dth, w_keep, hand, terr, error;
     // the lake parks of one wave: per droplet its park count and entry indices, per park the refused rest
     size_t w_park_n, w_park_k, w_park_rest;
+    size_t w_fin[3];   // the finish's gathered rows
     size_t w_offsets;  // long lists: each droplet's first compacted entry, and the wave's total
     int64_t ncell, nmetric, nslots, table_cap, table_slots, max_droplets, max_wave, wave_slots, cap;
 };

@@ -137,24 +137,24 @@ __device__ __forceinline__ void cp_wait()
 // key = the slot's cell (invalid past a list's end); the slots enter the stable sort in (droplet,
 // entry) order, so equal cells keep the serial order
 __global__ void ordered_keys_kernel(long long nslots, int cap, const int32_t *cell, const int64_t *count,
-                                    unsigned long long invalid, unsigned long long *keys, int32_t *vals)
+                                    SortKey invalid, SortKey *keys, int32_t *vals)
 {
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nslots; s += (long long)gridDim.x * blockDim.x) {
         const long long q = s / cap, k = s - q * cap;
-        keys[s] = k < count[q] ? (unsigned long long)cell[s] : invalid;
+        keys[s] = k < count[q] ? (SortKey)cell[s] : invalid;
         vals[s] = (int32_t)s;
     }
 }
 
 // the entries of a wave's lists compacted in (droplet, entry) order: entry k of droplet q goes to offsets[q] + k
 __global__ void ordered_compact_keys_kernel(long long nslots, int cap, const int32_t *cell, const int64_t *count,
-                                            const long long *offsets, unsigned long long *keys, int32_t *vals)
+                                            const long long *offsets, SortKey *keys, int32_t *vals)
 {
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nslots; s += (long long)gridDim.x * blockDim.x) {
         const long long q = s / cap, k = s - q * cap;
         if (k < count[q]) {
             const long long e = offsets[q] + k;
-            keys[e] = (unsigned long long)cell[s];
+            keys[e] = (SortKey)cell[s];
             vals[e] = (int32_t)s;
         }
     }
@@ -165,39 +165,24 @@ __global__ void entry_total_kernel(const int64_t *count, const long long *offset
     *total = nw > 0 ? offsets[nw - 1] + count[nw - 1] : 0;
 }
 
-// runstart: first slot of a (cell, droplet) run; segpos: position of a cell segment's first slot
-__global__ void ordered_flags_kernel(long long nslots, const unsigned long long *keys, const int32_t *vals, int cap,
-                                     unsigned long long invalid, int32_t *runstart, int32_t *segpos)
-{
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nslots; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long k = keys[i];
-        int rs = 0, sp = 0;
-        if (k != invalid) {
-            if (i == 0) {
-                rs = 1;
-            } else {
-                const bool newseg = keys[i - 1] != k;
-                rs = newseg || vals[i - 1] / cap != vals[i] / cap;
-                sp = newseg ? (int)i : 0;
-            }
-        }
-        runstart[i] = rs;
-        segpos[i] = sp;
-    }
-}
-
 // whether an entry reads the next one's cell live: an erosion (its floor) and a final deposit (its ceiling) do, a step
 // deposit and a lake park do not
 __device__ __forceinline__ bool reads_next(double delta, float vol) { return vol != -3.0f && (delta < 0.0 || vol < 0.0f); }
 
-__global__ void ordered_rank_kernel(long long nslots, const unsigned long long *keys, const int32_t *vals, int cap,
-                                    unsigned long long invalid, const int32_t *runscan, const int32_t *segscan,
-                                    const double *delta, const float *vol, const int64_t *count,
-                                    const CellTerr *terr, uint32_t epoch, EntryRec *rec)
+// One warp per 32 consecutive sorted slots.  An entry's rank is the number of droplets that start between its cell's
+// first slot and it: counted in the bits of the warp's slots, after those of the slots before them where their first
+// cell's run came in from there (looked back over 128 slots at a time: only a run longer than that goes round twice).
+// (Flags, two library scans and a pass over them: 22 us a wave in six launches at N_c = 1024; as here 7.4 in one.  The run's first warp walking all of it: 12.4, and 68 where runs reach thousands of entries.)
+__global__ void __launch_bounds__(256) ordered_rank_kernel(long long nslots, const SortKey *keys, const int32_t *vals, int cap,
+                                                           SortKey invalid, const double *delta, const float *vol,
+                                                           const int64_t *count, const CellTerr *terr, uint32_t epoch, EntryRec *rec)
 {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nslots; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long k = keys[i];
-        if (k == invalid) continue;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    // the record of sorted slot i: D distinct earlier droplets at its cell
+    auto emit = [&](long long i, SortKey k, uint32_t D) {
         const int32_t s = vals[i], q = s / cap, e = s - q * cap;
         const CellTerr t = terr[k];
         const float v = vol[s];
@@ -210,7 +195,6 @@ __global__ void ordered_rank_kernel(long long nslots, const unsigned long long *
         // the droplet's visits before and after this one are its neighbours in the sorted order
         const int32_t back = i > 0 && keys[i - 1] == k && vals[i - 1] / cap == q ? s - vals[i - 1] : 0;
         const int32_t fwd = i + 1 < nslots && keys[i + 1] == k && vals[i + 1] / cap == q ? vals[i + 1] - s : 0;
-        const uint32_t D = (uint32_t)(runscan[i] - runscan[segscan[i]]);  // distinct earlier droplets at the cell
         const bool reads = e + 1 < count[q] && reads_next(d, v);
         uint32_t f = (uint32_t)(back < APPLY_HIST ? back : APPLY_HIST);
         if (fwd == 0) f |= ENTRY_LAST;
@@ -226,6 +210,39 @@ __global__ void ordered_rank_kernel(long long nslots, const unsigned long long *
         r.flags = f;
         r.turn = epoch + D;
         rec[s] = r;
+    };
+    // whether slot i starts a droplet's visit to the cell of key k (the slot's own)
+    auto visit = [&](long long i, SortKey k) { return i == 0 || keys[i - 1] != k || vals[i - 1] / cap != vals[i] / cap; };
+    for (long long base = warp * 32; base < nslots; base += nwarps * 32) {
+        const long long i = base + lane;
+        const SortKey k = i < nslots ? keys[i] : invalid;
+        const unsigned cells = __ballot_sync(full, k != invalid && (i == 0 || keys[i - 1] != k));
+        const unsigned starts = __ballot_sync(full, k != invalid && visit(i, k));
+        const SortKey k0 = __shfl_sync(full, k, 0);
+        if (k0 == invalid) break;  // (the invalid slots come last)
+        uint32_t before = 0;  // droplets that start before this warp's slots at the cell whose run comes in
+        if (!(cells & 1u)) {
+            bool whole = true;
+            for (long long j0 = base - 128; whole; j0 -= 128) {
+                bool v[4], in[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const long long j = j0 + 32 * q + lane;
+                    in[q] = j >= 0 && keys[j] == k0;
+                    v[q] = in[q] && visit(j, k0);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    before += (uint32_t)__popc(__ballot_sync(full, v[q]));
+                    whole = __all_sync(full, in[q]) && whole;
+                }
+            }
+        }
+        if (k == invalid) continue;
+        const unsigned upto = full >> (31 - lane);
+        const unsigned own = cells & upto;  // the cells that start at or before this slot
+        const unsigned from = own ? full << (31 - __clz(own)) : full;
+        emit(i, k, (own ? 0u : before) + (uint32_t)__popc(starts & upto & from) - 1u);
     }
 }
 
@@ -241,23 +258,15 @@ __global__ void ordered_terrain_kernel(long long ncell, const double2 *L, const 
     }
 }
 
-struct MaxOp {
-    __device__ __forceinline__ int32_t operator()(const int32_t a, const int32_t b) const { return a > b ? a : b; }
-};
-
 size_t ordered_temp_bytes(long long nslots, long long max_wave)
 {
-    size_t a = 0, b = 0, c = 0, d = 0, x = 0;
+    size_t a = 0, d = 0, x = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, x, (int64_t *)nullptr, (long long *)nullptr, (int)max_wave);
-    cub::DeviceRadixSort::SortPairs(nullptr, a, (unsigned long long *)nullptr, (unsigned long long *)nullptr, (int32_t *)nullptr,
+    cub::DeviceRadixSort::SortPairs(nullptr, a, (SortKey *)nullptr, (SortKey *)nullptr, (int32_t *)nullptr,
                                     (int32_t *)nullptr, (int)nslots);
-    cub::DeviceScan::InclusiveSum(nullptr, b, (int32_t *)nullptr, (int32_t *)nullptr, (int)nslots);
-    cub::DeviceScan::InclusiveScan(nullptr, c, (int32_t *)nullptr, (int32_t *)nullptr, MaxOp{}, (int)nslots);
     cub::DeviceRadixSort::SortPairs(nullptr, d, (uint32_t *)nullptr, (uint32_t *)nullptr, (int32_t *)nullptr, (int32_t *)nullptr,
                                     (int)(max_wave * LAKE_PARKS));
-    size_t m = a > b ? a : b;
-    m = m > c ? m : c;
-    m = m > d ? m : d;
+    const size_t m = a > d ? a : d;
     return m > x ? m : x;
 }
 
@@ -644,11 +653,11 @@ __global__ void __launch_bounds__(32) ordered_apply_kernel(const OrderedArgs a)
 // gathers what its entry adds into arrays in sorted order (one thread a slot, all loads in flight at
 // once); then one thread a cell sums its run of those arrays in order (contiguous reads).
 // ---------------------------------------------------------------------------
-__global__ void ordered_gather_kernel(const OrderedArgs a, long long nslots, const unsigned long long *keys, const int32_t *vals,
-                                      unsigned long long invalid, FinishRows g)
+__global__ void ordered_gather_kernel(const OrderedArgs a, long long nslots, const SortKey *keys, const int32_t *vals,
+                                      SortKey invalid, FinishRows g)
 {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nslots; i += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long key = keys[i];
+        const SortKey key = keys[i];
         if (key == invalid) continue;
         const int32_t s = vals[i], q = s / a.cap;
         const bool active = !a.mask || a.mask[key] == PGE_MASK_ACTIVE;
@@ -661,85 +670,121 @@ __global__ void ordered_gather_kernel(const OrderedArgs a, long long nslots, con
     }
 }
 
-// One warp per 32 consecutive sorted slots; the warp walks every cell run that starts in its slots, 32
-// entries at a time: the lanes load a step's rows at once, then every lane adds them in lane order (the
-// float64 sums in the serial order, the additions shuffled out of the lanes), the integer totals per lane
-constexpr int FINISH_THREADS = 256, FINISH_WARPS = FINISH_THREADS / 32;
+// One warp per 32 consecutive sorted slots, for the cell runs that start there.  The rows of 64 slots are laid out as
+// float64 in shared memory; a run that ends within them is added by the lane of its first slot, all of a warp's runs at
+// once.  A longer one is walked by the whole warp, 32 entries at a time (the next window's rows read while this one is
+// added), four lanes adding one sum each -- the discharge, the two momentum tracks and the stockpile.  Either way a sum
+// is added in slot order, the serial order.  (An entry that adds nothing to a sum adds 0, which leaves it as it is: the
+// sums start at +0 and so are never -0.)
+//
+// Bound by the latency of a run's reads and the float64 adds of the longest.  Every run walked by the warp, one after
+// another: 36.6 us a wave at N_c = 1024, 81-104 at N_c = 128 where hundreds of a wave's droplets cross a cell; 8.1 and 30.
+constexpr int FINISH_THREADS = 256, FINISH_WARPS = FINISH_THREADS / 32, FINISH_PITCH = 68;  // (no two sums' reads share a bank)
 
-__global__ void __launch_bounds__(FINISH_THREADS) ordered_finish_kernel(const OrderedArgs a, long long nslots, const unsigned long long *keys,
-                                      unsigned long long invalid, FinishRows g)
+struct FinishRow {
+    float v, m0, m1;
+    double kp;
+};
+
+__global__ void __launch_bounds__(FINISH_THREADS) ordered_finish_kernel(const OrderedArgs a, long long nslots, const SortKey *keys,
+                                                                        SortKey invalid, FinishRows g)
 {
-    // each warp's window of its run, read in order by every lane (broadcast reads: the loads of later slots
-    // go out ahead of the float64 sums, which keep the serial order)
-    __shared__ float sv[FINISH_WARPS][32], sa[FINISH_WARPS][32], sb[FINISH_WARPS][32];
-    __shared__ double sk[FINISH_WARPS][32];
+    __shared__ double win[FINISH_WARPS][4][FINISH_PITCH];
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    double(*w)[FINISH_PITCH] = win[threadIdx.x >> 5];
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    auto row = [&](long long j) { return FinishRow{g.v[j], g.m0[j], g.m1[j], g.kp[j]}; };
+    auto lay = [&](int at, const FinishRow &r) {
+        const bool step = r.v > 0.0f;  // a step of volume > 0 on an active cell (gathered as 0 otherwise)
+        w[0][at] = step ? (double)r.v : 0.0;
+        w[1][at] = step ? (double)r.m0 : 0.0;
+        w[2][at] = step ? (double)r.m1 : 0.0;
+        w[3][at] = r.kp >= 0.0 ? r.kp : 0.0;
+    };
+    const FinishRow none{0.0f, 0.0f, 0.0f, -1.0};
+    // a touched cell's net change to the accumulators and its packed samples (particle.py:1005-1009)
+    auto settle = [&](long long c) {
+        const unsigned long long *hw = reinterpret_cast<const unsigned long long *>(a.hand + c);
+        const double acc = hand_acc(hw[0], hw[1]);
+        a.acc4[4 * c] = acc;
+        if (!a.mask || a.mask[c] == PGE_MASK_ACTIVE) {
+            const float surf = (float)(a.L[c].x + acc);
+            a.A[c].x = surf;
+            const double sd = a.sediment[c] + acc;
+            a.B[c].z = (float)(sd > 0.0 ? sd : 0.0);
+            // the route flag follows the live surface; a lake cell stays a lake cell (particle.py:1010-1012)
+            if (a.R && a.R[c].y < 1.5f) a.R[c].y = a.R[c].x != surf ? 1.0f : 0.0f;
+        }
+    };
     for (long long base = warp * 32; base < nslots; base += nwarps * 32) {
-        const long long i = base + lane;
-        const unsigned long long ki = i < nslots ? keys[i] : invalid;
-        const bool head = ki != invalid && (i == 0 || keys[i - 1] != ki);
-        unsigned heads = __ballot_sync(full, head);
-        while (heads) {
-            const int hl = __ffs(heads) - 1;
-            heads &= heads - 1;
-            const unsigned long long key = __shfl_sync(full, ki, hl);
-            const long long c = (long long)key;
+        const long long i = base + lane, i2 = i + 32;
+        const SortKey k0 = i < nslots ? keys[i] : invalid, k1 = i2 < nslots ? keys[i2] : invalid;
+        SortKey before = __shfl_up_sync(full, k0, 1);
+        if (lane == 0) before = base > 0 ? keys[base - 1] : ~k0;
+        SortKey mid = __shfl_up_sync(full, k1, 1);
+        const SortKey last0 = __shfl_sync(full, k0, 31);
+        if (lane == 0) mid = last0;
+        const bool head = k0 != invalid && before != k0;
+        const unsigned heads = __ballot_sync(full, head);
+        if (!heads) continue;
+        // bit b: slot base + b does not go on with the run of the slot before it
+        const unsigned long long ends = (unsigned long long)__ballot_sync(full, before != k0) | ((unsigned long long)__ballot_sync(full, mid != k1) << 32);
+        const unsigned long long rest = lane < 63 ? ends >> (lane + 1) : 0ull;
+        const int len = rest ? __ffsll((long long)rest) : 0;  // 0: the run goes on past the window
+        lay(lane, k0 != invalid ? row(i) : none);
+        lay(32 + lane, k1 != invalid ? row(i2) : none);
+        __syncwarp();
+        if (head && len) {
+            const long long c = (long long)k0;
             double *accp = a.acc4 + 4 * c;
             double tq = accp[1], ta = accp[2], tb = accp[3], pd = a.pend[c];
-            for (long long j0 = base + hl;; j0 += 32) {
-                const long long j = j0 + lane;
-                const bool in = j < nslots && keys[j] == key;
-                float v = 0.0f, m0 = 0.0f, m1 = 0.0f;
-                double kp = -1.0;
-                if (in) {
-                    v = g.v[j];
-                    m0 = g.m0[j];
-                    m1 = g.m1[j];
-                    kp = g.kp[j];
+            for (int t = lane; t < lane + len; t++) {
+                tq += w[0][t];
+                ta += w[1][t];
+                tb += w[2][t];
+                pd += w[3][t];
+            }
+            accp[1] = tq;
+            accp[2] = ta;
+            accp[3] = tb;
+            a.pend[c] = pd;
+            settle(c);
+        }
+        __syncwarp();
+        unsigned longer = __ballot_sync(full, head && !len);  // (at most the last run)
+        while (longer) {
+            const int hl = __ffs(longer) - 1;
+            longer &= longer - 1;
+            const SortKey key = __shfl_sync(full, k0, hl);
+            const long long c = (long long)key;
+            double *mine = lane < 3 ? a.acc4 + 4 * c + 1 + lane : a.pend + c;  // this lane's sum (the first four lanes)
+            double sum = lane < 4 ? *mine : 0.0;
+            long long j = base + hl + lane;
+            bool in = j < nslots && keys[j] == key;
+            FinishRow r = in ? row(j) : none;
+            while (true) {
+                const int n = __popc(__ballot_sync(full, in));  // the run covers a prefix of the lanes (keys are sorted)
+                lay(lane, r);
+                if (n == 32) {
+                    j += 32;
+                    in = j < nslots && keys[j] == key;
+                    r = in ? row(j) : none;
                 }
-                // the run covers a prefix of the lanes (keys are sorted)
-                const int n = __popc(__ballot_sync(full, in));
-                sv[wib][lane] = v;
-                sa[wib][lane] = m0;
-                sb[wib][lane] = m1;
-                sk[wib][lane] = kp;
                 __syncwarp();
-#pragma unroll 4
-                for (int t = 0; t < n; t++) {
-                    const float vt = sv[wib][t];
-                    const float at = sa[wib][t];
-                    const float bt = sb[wib][t];
-                    const double kt = sk[wib][t];
-                    if (vt > 0.0f) {  // a step of volume > 0 on an active cell (gathered as 0 otherwise)
-                        tq += (double)vt;
-                        ta += (double)at;
-                        tb += (double)bt;
-                    }
-                    if (kt >= 0.0) pd += kt;
+                const double *mw = w[lane & 3];
+                if (n == 32) {
+#pragma unroll 8
+                    for (int t = 0; t < 32; t++) sum += mw[t];
+                } else {
+                    for (int t = 0; t < n; t++) sum += mw[t];
                 }
                 __syncwarp();  // every lane has read the window before the next one is written
                 if (n < 32) break;
             }
-            if (lane == 0) {
-                accp[1] = tq;
-                accp[2] = ta;
-                accp[3] = tb;
-                a.pend[c] = pd;
-                const unsigned long long *hw = reinterpret_cast<const unsigned long long *>(a.hand + c);
-                const double acc = hand_acc(hw[0], hw[1]);
-                accp[0] = acc;
-                if (!a.mask || a.mask[c] == PGE_MASK_ACTIVE) {
-                    const float surf = (float)(a.L[c].x + acc);
-                    a.A[c].x = surf;
-                    const double sd = a.sediment[c] + acc;
-                    a.B[c].z = (float)(sd > 0.0 ? sd : 0.0);
-                    // the route flag follows the live surface; a lake cell stays a lake cell (particle.py:1010-1012)
-                    if (a.R && a.R[c].y < 1.5f) a.R[c].y = a.R[c].x != surf ? 1.0f : 0.0f;
-                }
-            }
+            if (lane < 4) *mine = sum;
+            if (lane == 0) settle(c);
         }
     }
 }
@@ -788,13 +833,8 @@ cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st)
     tb = w.temp_bytes;
     e = cub::DeviceRadixSort::SortPairs(w.temp, tb, w.keys_in, w.keys_out, w.vals_in, w.vals_out, (int)nslots, 0, w.end_bit, st);
     if (e != cudaSuccess) return e;
-    ordered_flags_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.keys_out, w.vals_out, w.cap, w.invalid, w.runstart, w.segpos);
-    tb = w.temp_bytes;
-    if ((e = cub::DeviceScan::InclusiveSum(w.temp, tb, w.runstart, w.runscan, (int)nslots, st)) != cudaSuccess) return e;
-    tb = w.temp_bytes;
-    if ((e = cub::DeviceScan::InclusiveScan(w.temp, tb, w.segpos, w.segscan, MaxOp{}, (int)nslots, st)) != cudaSuccess) return e;
-    ordered_rank_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.keys_out, w.vals_out, w.cap, w.invalid, w.runscan, w.segscan,
-                                                          w.a.delta, w.a.vol, w.a.count, w.a.terr, w.a.epoch, const_cast<EntryRec *>(w.a.rec));
+    ordered_rank_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.keys_out, w.vals_out, w.cap, w.invalid, w.a.delta, w.a.vol, w.a.count,
+                                                          w.a.terr, w.a.epoch, const_cast<EntryRec *>(w.a.rec));
     const bool lake = w.a.lakes && w.a.R;
     const int blocks = (int)w.nw;  // a warp per droplet, the earlier droplets' blocks first
     if (w.a.ecap && lake)
@@ -805,12 +845,11 @@ cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st)
         ordered_apply_kernel<false, true><<<blocks, 32, 0, st>>>(w.a);
     else
         ordered_apply_kernel<false, false><<<blocks, 32, 0, st>>>(w.a);
-    // the sort's input keys and the scans' buffers are free again: the gathered rows live there
     FinishRows g;
-    g.v = reinterpret_cast<float *>(w.runstart);
-    g.m0 = reinterpret_cast<float *>(w.segpos);
-    g.m1 = reinterpret_cast<float *>(w.runscan);
-    g.kp = reinterpret_cast<double *>(w.keys_in);
+    g.v = w.fin[0];
+    g.m0 = w.fin[1];
+    g.m1 = w.fin[2];
+    g.kp = reinterpret_cast<double *>(w.keys_in);  // (the sort's input keys are free again)
     ordered_gather_kernel<<<grid_for(nslots), 256, 0, st>>>(w.a, nslots, w.keys_out, w.vals_out, w.invalid, g);
     ordered_finish_kernel<<<grid_for(nslots, FINISH_THREADS), FINISH_THREADS, 0, st>>>(w.a, nslots, w.keys_out, w.invalid, g);
     return cudaPeekAtLastError();
