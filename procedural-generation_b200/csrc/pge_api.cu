@@ -381,10 +381,15 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
                                          : s->route ? droplet_blocks_per_sm_f64_route(32, false)
                                          : p->precision == PGE_PREC_F64 ? droplet_blocks_per_sm_f64(32, 1, false)
                                                                       : droplet_blocks_per_sm_f32(32, 1, false));
-            // the plain float64 record-only trace also comes in a 128-register build: more warps resident,
-            // so a wave that fits runs one droplet per warp (no lane waits on another droplet's branches)
-            const bool plain64 = !lateral && !s->route && p->precision == PGE_PREC_F64;
-            const long long rec_warps_lean = plain64 ? (long long)sm_count() * droplet_blocks_per_sm_f64(32, 2, false) : 0;
+            // a float64 wave whose droplets fit the GPU as one warp each (2368) takes the trace of one warp a droplet:
+            // waves of 2048: 184 against 305 us (N = 512 sphere), 297 against 493 with lakes, 316 against 505 with
+            // banks; of 4096: 315 against 303, 369 against 544, 329 against 539; of 8192: 523 against 352, 486 against
+            // 646 (some 6000 with lakes).  A thread's step with a route or banks is that much longer, so there the
+            // line lies at twice the residents.
+            const long long warp_waves = p->precision == PGE_PREC_F64 && p->trace_lanes == 0
+                                             ? (long long)sm_count() * trace_blocks_per_sm_f64(s->route != nullptr, lateral) *
+                                                   (s->route || lateral ? 2 : 1)
+                                             : 0;
             int ebits = 1;
             while ((1LL << ebits) <= wave) ebits++;
             long long ebase = 0;
@@ -394,23 +399,22 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
                 a.rec_base = a.d_begin;
                 a.counter = ctr + (w & 1);
                 a.counter_next = ctr + ((w + 1) & 1);
-                // a small wave is latency-bound: spread it over every SM (one or two warps each)
-                // a wave's trace is latency-bound (each droplet is a serial chain of steps): give each
-                // warp as few droplets as keeps every warp resident, so lanes do not wait on each
-                // other's branches
                 const long long nd = a.d_end - a.d_begin;
-                long long lanes = p->trace_lanes > 0 ? p->trace_lanes : (nd + rec_warps - 1) / rec_warps;
-                a.minb = 1;
-                if (p->trace_lanes == 0 && plain64 && nd <= rec_warps_lean) {
-                    lanes = 1;
-                    a.minb = 2;
+                if (nd <= warp_waves) {
+                    e = launch_trace_f64(a, st);
+                } else {
+                    // a wave's trace is latency-bound (each droplet is a serial chain of steps): give each
+                    // warp as few droplets as keeps every warp resident, so lanes do not wait on each
+                    // other's branches
+                    const long long lanes = p->trace_lanes > 0 ? p->trace_lanes : (nd + rec_warps - 1) / rec_warps;
+                    a.minb = 1;
+                    a.lanes = (int)(lanes < 1 ? 1 : (lanes > 32 ? 32 : lanes));
+                    const int tpb = 32;
+                    long long blocks = (nd + a.lanes - 1) / a.lanes;
+                    if (blocks * tpb > droplet_slots()) blocks = droplet_slots() / tpb;  // no tables: the GPU's resident threads
+                    e = p->precision == PGE_PREC_F64 ? launch_droplets_f64(a, (int)blocks, tpb, st)
+                                                     : launch_droplets_f32(a, (int)blocks, tpb, st);
                 }
-                a.lanes = (int)(lanes < 1 ? 1 : (lanes > 32 ? 32 : lanes));
-                const int tpb = 32;
-                long long blocks = (nd + a.lanes - 1) / a.lanes;
-                if (blocks * tpb > droplet_slots()) blocks = droplet_slots() / tpb;  // no tables: the GPU's resident threads
-                e = p->precision == PGE_PREC_F64 ? launch_droplets_f64(a, (int)blocks, tpb, st)
-                                                 : launch_droplets_f32(a, (int)blocks, tpb, st);
                 if (e != cudaSuccess) return cuda_fail(e, "droplet kernel");
                 ow.nw = nd;
                 oa.nw = ow.nw;

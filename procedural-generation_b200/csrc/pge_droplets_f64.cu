@@ -3,21 +3,39 @@
 #define PGE_REAL double
 #define PGE_VARIANT f64
 #include "pge_droplets.cuh"
+#include "pge_trace.cuh"
 
 namespace pge {
 cudaError_t launch_droplets_f64(const DropArgs &a, int blocks, int threads, cudaStream_t st)
 {
     if (a.p.lateral_rate > 0.0) return launch_droplets_f64_lateral(a, blocks, threads, st);
     if (a.R) return launch_droplets_f64_route(a, blocks, threads, st);
-    if (!a.ledger && a.minb >= 2)  // record only, at most 128 registers: a wave's droplets one per warp
-        f64::droplet_kernel<2, false><<<blocks, threads, 0, st>>>(a);
-    else if (!a.ledger)
+    if (!a.ledger)
         f64::droplet_kernel<1, false><<<blocks, threads, 0, st>>>(a);
     else if (a.minb >= 2)
         f64::droplet_kernel<2, true><<<blocks, threads, 0, st>>>(a);
     else
         f64::droplet_kernel<1, true><<<blocks, threads, 0, st>>>(a);
     return cudaPeekAtLastError();
+}
+namespace {
+typedef void (*TraceKernel)(const DropArgs);
+TraceKernel trace_variant(bool route, bool lateral)
+{
+    return route ? (lateral ? f64::trace_kernel<true, true> : f64::trace_kernel<true, false>)
+                 : (lateral ? f64::trace_kernel<false, true> : f64::trace_kernel<false, false>);
+}
+}  // namespace
+cudaError_t launch_trace_f64(const DropArgs &a, cudaStream_t st)
+{
+    trace_variant(a.R != nullptr, a.p.lateral_rate > 0.0)<<<(int)(a.d_end - a.d_begin), 32, 0, st>>>(a);
+    return cudaPeekAtLastError();
+}
+int trace_blocks_per_sm_f64(bool route, bool lateral)
+{
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, trace_variant(route, lateral), 32, 0) != cudaSuccess) return 1;
+    return n > 0 ? n : 1;
 }
 cudaError_t launch_droplets_f64_route(const DropArgs &a, int blocks, int threads, cudaStream_t st)
 {
@@ -73,8 +91,7 @@ int droplet_blocks_per_sm_f64_tape(int threads)
 int droplet_blocks_per_sm_f64(int threads, int minb, bool ledger)
 {
     int n = 0;
-    cudaError_t e = !ledger     ? (minb >= 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f64::droplet_kernel<2, false>, threads, 0)
-                                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f64::droplet_kernel<1, false>, threads, 0))
+    cudaError_t e = !ledger     ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f64::droplet_kernel<1, false>, threads, 0)
                     : minb >= 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f64::droplet_kernel<2, true>, threads, 0)
                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f64::droplet_kernel<1, true>, threads, 0);
     if (e != cudaSuccess) return 1;

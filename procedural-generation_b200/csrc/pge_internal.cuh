@@ -136,6 +136,9 @@ struct DropArgs {
 // launchers of the two precisions (separate translation units: the float64
 // one is compiled without FMA contraction so it rounds like the reference)
 cudaError_t launch_droplets_f64(const DropArgs &a, int blocks, int threads, cudaStream_t st);
+// the exact pass's trace, one warp a droplet (pge_trace.cuh): float64, record only
+cudaError_t launch_trace_f64(const DropArgs &a, cudaStream_t st);
+int trace_blocks_per_sm_f64(bool route, bool lateral);
 cudaError_t launch_droplets_f64_tape(const DropArgs &a, int blocks, int threads, cudaStream_t st);
 cudaError_t launch_droplets_f64_route(const DropArgs &a, int blocks, int threads, cudaStream_t st);
 cudaError_t launch_droplets_f64_lateral(const DropArgs &a, int blocks, int threads, cudaStream_t st);
