@@ -382,7 +382,7 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
                                          : p->precision == PGE_PREC_F64 ? droplet_blocks_per_sm_f64(32, 1, false)
                                                                       : droplet_blocks_per_sm_f32(32, 1, false));
             // a float64 wave whose droplets fit the GPU as one warp each (2368) takes the trace of one warp a droplet:
-            // waves of 2048: 184 against 305 us (N = 512 sphere), 297 against 493 with lakes, 316 against 505 with
+            // waves of 2048: 184 against 305 us (N_c = 1024), 297 against 493 with lakes, 316 against 505 with
             // banks; of 4096: 315 against 303, 369 against 544, 329 against 539; of 8192: 523 against 352, 486 against
             // 646 (some 6000 with lakes).  A thread's step with a route or banks is that much longer, so there the
             // line lies at twice the residents.

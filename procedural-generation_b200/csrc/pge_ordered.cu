@@ -172,7 +172,8 @@ __device__ __forceinline__ bool reads_next(double delta, float vol) { return vol
 // One warp per 32 consecutive sorted slots.  An entry's rank is the number of droplets that start between its cell's
 // first slot and it: counted in the bits of the warp's slots, after those of the slots before them where their first
 // cell's run came in from there (looked back over 128 slots at a time: only a run longer than that goes round twice).
-// (Flags, two library scans and a pass over them: 22 us a wave in six launches at N_c = 1024; as here 7.4 in one.  The run's first warp walking all of it: 12.4, and 68 where runs reach thousands of entries.)
+// (Flags, two library scans and a pass over them: 22 us a wave in six launches at N_c = 1024; as here 7.4 in one.
+// The run's first warp walking all of it: 12.4, and 68 where runs reach thousands of entries.)
 __global__ void __launch_bounds__(256) ordered_rank_kernel(long long nslots, const SortKey *keys, const int32_t *vals, int cap,
                                                            SortKey invalid, const double *delta, const float *vol,
                                                            const int64_t *count, const CellTerr *terr, uint32_t epoch, EntryRec *rec)

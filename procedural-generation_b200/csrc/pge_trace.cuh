@@ -6,7 +6,7 @@
 //
 // What bounds a wave is one droplet's serial chain of steps.  On a thread of its own a step is one long in-order run
 // of ~1000 instructions, eleven divisions and roots of the path and seven of the mass transfer among them (305 us a
-// wave of 2048 droplets on the N = 512 sphere, some 6000 cycles a step).  But the path does not depend on the load:
+// wave of 2048 droplets on the N_c = 1024 sphere, some 6000 cycles a step).  But the path does not depend on the load:
 // positions, directions and the volume are decided by the frozen surface alone, and the load only adds two ways to
 // die, both at sea.  So a warp
 //   1. walks the path up to TB steps ahead.  All lanes walk the same path; where a step needs several like things at
@@ -18,8 +18,8 @@
 //   3. runs the load's own recurrence over the steps in order (a handful of operations and the quotient by the
 //      evaporation, from its reciprocal), which also finds a death at sea that ends the path early;
 //   4. writes the entries, a lane an entry.
-// At sea the walk goes only TB_SEA steps ahead, since the load may end it.  Measured, a wave: 184 us (N = 512 sphere),
-// 297 with lakes (a thread a droplet: 493), 316 with banks (505), 82 where N = 32 (102).  A step's walk is ~2900
+// At sea the walk goes only TB_SEA steps ahead, since the load may end it.  Measured, a wave: 184 us (N_c = 1024 sphere),
+// 297 with lakes (a thread a droplet: 493), 316 with banks (505), 82 where N_c = 32 (102).  A step's walk is ~2900
 // cycles of it, ~800 of them the view's loads and ~1300 the five divisions and roots with their shuffles.
 //
 // The lanes agree on everything they walk, so one lane keeps the batch's record; a record stored by all 32 at once is
