@@ -221,8 +221,9 @@ typedef struct PgeParams {
     int32_t use_erode_cap;   /* slope_limit_erode > 0: erode_cap passed to pge_trace_apply */
     int32_t threads_per_block; /* 0 = default */
     int32_t blocks_per_sm;     /* 0 = occupancy maximum */
-    int32_t trace_lanes;       /* ordered apply: droplets per warp in each wave's trace; 0 = as few as keep
-                                  every warp of the wave resident (fastest alone), up to 32 (smallest
+    int32_t trace_lanes;       /* ordered apply: droplets per warp in each wave's trace, a thread each; 0 = a whole
+                                  warp a droplet where the wave fits the GPU that way (float64), else as few as
+                                  keep every warp of the wave resident (fastest alone); up to 32 (smallest
                                   footprint, for passes of several worlds running at once) */
     int32_t apply_lanes;       /* 0..32, accepted and without effect: the ordered apply runs one droplet per warp
                                   (lanes waiting on different hand-offs would take turns) */
