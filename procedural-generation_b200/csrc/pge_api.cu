@@ -338,6 +338,7 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
             oa.p = *p;
             oa.stats = stats;
             oa.error = ws_ptr<int>(ws, lay.error);
+            oa.ticket = ws_ptr<unsigned int>(ws, lay.error) + 32;  // (a line of its own)
             ParkWave pw{};
             if (parks) {
                 a.park_n = ws_ptr<int32_t>(ws, lay.w_park_n);

@@ -137,8 +137,9 @@ __device__ __forceinline__ void cp_wait()
 // key = the slot's cell (invalid past a list's end); the slots enter the stable sort in (droplet,
 // entry) order, so equal cells keep the serial order
 __global__ void ordered_keys_kernel(long long nslots, int cap, const int32_t *cell, const int64_t *count,
-                                    SortKey invalid, SortKey *keys, int32_t *vals)
+                                    SortKey invalid, SortKey *keys, int32_t *vals, unsigned int *ticket)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nslots; s += (long long)gridDim.x * blockDim.x) {
         const long long q = s / cap, k = s - q * cap;
         keys[s] = k < count[q] ? (SortKey)cell[s] : invalid;
@@ -148,8 +149,9 @@ __global__ void ordered_keys_kernel(long long nslots, int cap, const int32_t *ce
 
 // the entries of a wave's lists compacted in (droplet, entry) order: entry k of droplet q goes to offsets[q] + k
 __global__ void ordered_compact_keys_kernel(long long nslots, int cap, const int32_t *cell, const int64_t *count,
-                                            const long long *offsets, SortKey *keys, int32_t *vals)
+                                            const long long *offsets, SortKey *keys, int32_t *vals, unsigned int *ticket)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nslots; s += (long long)gridDim.x * blockDim.x) {
         const long long q = s / cap, k = s - q * cap;
         if (k < count[q]) {
@@ -530,6 +532,10 @@ __device__ __forceinline__ void droplet_end(const OrderedArgs &a, const Walk &w,
 // One warp a droplet: every lane runs the droplet's entries (the same values in all lanes), the lanes share the
 // copies of its records and the statistics of 32 entries at a time.
 //
+// A block takes the next droplet by a ticket, so the droplets it can wait for -- the earlier ones -- have all started,
+// in whatever order the GPU starts a wave's blocks and however few of them it holds at once (of one-warp blocks 32 a
+// multiprocessor): the earliest droplet that has not ended waits for nobody.
+//
 // Bound by the instructions of one entry on one warp (~110, 215-235 ns; 2048 droplets at work at once: 405), not
 // by memory.  What each choice measured, ns an entry without a wait: hand-off words read into registers ahead of
 // their use 430 (the compiler's wait for any shared-memory read then waits for them too), by asynchronous copies
@@ -548,7 +554,9 @@ __global__ void __launch_bounds__(32) ordered_apply_kernel(const OrderedArgs a)
     __shared__ float2 route[LAKE ? REC_RING : 1];
     const PgeParams &p = a.p;
     const int lane = threadIdx.x;
-    const long long q = blockIdx.x;
+    unsigned int mine = 0;
+    if (lane == 0) mine = atomicAdd(a.ticket, 1u);
+    const long long q = __shfl_sync(FULL, mine, 0);
     const int K = (int)a.count[q];
     if (K <= 0) {
         if (lane == 0) a.dth[q] = -1;
@@ -875,10 +883,11 @@ cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st)
         if ((e = cudaMemcpyAsync(&total, w.offsets + w.nw, sizeof(long long), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
         ordered_compact_keys_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.cap, w.a.cell, w.a.count, w.offsets, w.keys_in,
-                                                                      w.vals_in);
+                                                                      w.vals_in, w.a.ticket);
         nslots = total;
     } else {
-        ordered_keys_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.cap, w.a.cell, w.a.count, w.invalid, w.keys_in, w.vals_in);
+        ordered_keys_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.cap, w.a.cell, w.a.count, w.invalid, w.keys_in, w.vals_in,
+                                                              w.a.ticket);
     }
     tb = w.temp_bytes;
     e = cub::DeviceRadixSort::SortPairs(w.temp, tb, w.keys_in, w.keys_out, w.vals_in, w.vals_out, (int)nslots, 0, w.end_bit, st);
@@ -886,7 +895,7 @@ cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st)
     ordered_rank_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.keys_out, w.vals_out, w.cap, w.invalid, w.a.delta, w.a.vol, w.a.count,
                                                           w.a.terr, w.a.epoch, const_cast<EntryRec *>(w.a.rec));
     const bool lake = w.a.lakes && w.a.R;
-    const int blocks = (int)w.nw;  // a warp per droplet, the earlier droplets' blocks first
+    const int blocks = (int)w.nw;  // a warp per droplet
     if (w.a.ecap && lake)
         ordered_apply_kernel<true, true><<<blocks, 32, 0, st>>>(w.a);
     else if (w.a.ecap)

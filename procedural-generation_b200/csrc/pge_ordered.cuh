@@ -70,6 +70,7 @@ struct OrderedArgs {
     PgeParams p;
     PgeStats *stats;
     int *error;
+    unsigned int *ticket;  // droplets of the wave taken so far (zeroed by the keys kernel)
     // lake parks (nullptr: off): per droplet its park count, per park (LAKE_PARKS a droplet) the rest its lake
     // had no room for, added to the droplet's leftover load in list order
     const int32_t *park_n;
