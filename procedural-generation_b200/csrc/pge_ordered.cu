@@ -57,15 +57,8 @@ inline int grid_for(long long n, int threads = 256)
     return (int)(b < 1 ? 1 : (b > 1048576 ? 1048576 : b));
 }
 
-constexpr int kSpinLimit = 1 << 24;  // ~ seconds of polling: far beyond any real hand-off
-// a waiting warp sleeps PGE_POLL_SLEEP_NS after every PGE_POLL_EVERY polls (a power of two)
-#ifndef PGE_POLL_EVERY
-#define PGE_POLL_EVERY 256
-#endif
-#ifndef PGE_POLL_SLEEP_NS
-#define PGE_POLL_SLEEP_NS 32
-#endif
-static_assert((PGE_POLL_EVERY & (PGE_POLL_EVERY - 1)) == 0, "poll interval: a power of two");
+constexpr int kSpinLimit = 1 << 24;  // ~ seconds of looks and sleeps: far beyond any real hand-off
+constexpr int POLL_EVERY = 256;      // looks between two at whether another wait has given up (a power of two)
 
 // A cell's hand-off word: 16 bytes, two 8-byte halves (acc low 32 bits | count << 32) and (acc high
 // 32 bits | count << 32), where acc is the live net change and count the hand-off counter.  Each
@@ -397,13 +390,11 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 // records of a droplet's list on chip: the chunk being applied, the next two and the one before (a power of two)
 constexpr int REC_RING = 128;
-// a waiting warp whose turn is n droplets away sleeps n * BACK_NS (at most BACK_MAX of them) between its looks
-#ifndef PGE_BACK_NS
-#define PGE_BACK_NS 64
-#endif
-#ifndef PGE_BACK_MAX
-#define PGE_BACK_MAX 16
-#endif
+// a waiting warp whose turn is n droplets away sleeps n - 1 times BACK_NS (at most BACK_MAX of them; a hand-off takes
+// several) between its looks.  A wave whose droplets all cross one cell, us a pass at 2048 / 4096 / 8192 / 32,768
+// droplets: at most 16 of them 3290 / 9406 / 22,843 / 103,940 (the looks then hold up the hand-offs), 256 of them
+// 3040 / 5710 / 11,110 / 43,510; waves spread over the terrain are the same with either (2048 droplets: 832, 825).
+constexpr uint32_t BACK_NS = 64, BACK_MAX = 256;
 
 template <int N>
 struct Int {
@@ -624,20 +615,25 @@ __global__ void __launch_bounds__(32) ordered_apply_kernel(const OrderedArgs a)
         ulonglong2 wc;
         const bool late = !ok;
         if (late) {
-            for (int i = 0; !ok; i++) {
+            for (int i = 0, waited = 0; !ok; i++) {
                 if (need_a && !hand_ready(wa.x, wa.y, A.turn)) hand_load(a.hand + A.cell, wa.x, wa.y);
                 hand_load(a.hand + B.cell, wb.x, wb.y);
                 hand_load(a.hand + C.cell, wc.x, wc.y);
                 const bool ok_a = !need_a || hand_ready(wa.x, wa.y, A.turn);
                 ok = ok_a && (!need_b || hand_ready(wb.x, wb.y, B.turn));
                 if ((i & 3) == 3 && !ok) {
-                    // droplets still to come before the one that hands the cell to this one: look less often, so that the
-                    // waiting warps leave their issue slots to the ones at work
+                    // droplets still to come before the one that hands the cell to this one: sleep the least time they
+                    // take, so that the looks of all who wait for one cell do not hold up the hand-offs on it
                     const uint32_t at = (uint32_t)((ok_a ? wb.x : wa.x) >> 32), want = ok_a ? B.turn : A.turn;
                     const uint32_t away = want - ((int32_t)(at - a.epoch) < 0 ? a.epoch : at);
-                    if (away > 1) __nanosleep((away < PGE_BACK_MAX ? away - 1 : PGE_BACK_MAX) * PGE_BACK_NS);
-                    if ((i & (PGE_POLL_EVERY - 1)) == PGE_POLL_EVERY - 1 && (i >= kSpinLimit || *(volatile int *)a.error)) {
-                        if (i >= kSpinLimit) atomicExch(a.error, 1);
+                    if (away > 1) {
+                        const uint32_t n = away < BACK_MAX ? away - 1 : BACK_MAX;
+                        __nanosleep(n * BACK_NS);
+                        waited += (int)(n >> 3);  // (a look takes about eight of them)
+                    }
+                    waited += 4;
+                    if (waited >= kSpinLimit || ((i & (POLL_EVERY - 1)) == POLL_EVERY - 1 && *(volatile int *)a.error)) {
+                        if (waited >= kSpinLimit) atomicExch(a.error, 1);
                         return false;  // this wait, or another one, gave up
                     }
                 }

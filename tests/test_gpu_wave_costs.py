@@ -1,0 +1,44 @@
+"""Costs of the exact pass that have to grow with the wave and no faster,
+measured on the device as ratios within one process (both sides the same
+kernel on the same GPU, the best of three passes each)."""
+import numpy as np
+import pytest
+import torch
+
+from pgerosion import maps as gm
+from tests.parity_cases import gpu_window, window_world
+
+pytestmark = pytest.mark.gpu
+
+
+def _kernel_us(run, kernel, tries=3):
+    """Device time of the kernels whose name holds ``kernel`` in one call of ``run``, the best of ``tries``."""
+    from torch.profiler import ProfilerActivity, profile
+
+    run()
+    best = float("inf")
+    for _ in range(tries):
+        torch.cuda.synchronize()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            run()
+            torch.cuda.synchronize()
+        us = sum(e.device_time_total for e in prof.key_averages() if kernel in e.key)
+        assert us > 0.0, kernel
+        best = min(best, us)
+    return best
+
+
+def _crowded(P, max_steps, evap_rate=0.01):
+    """A pass of one wave whose droplets all start on one cell of a bowl's floor."""
+    arr, params = window_world("closed", N=24)
+    ep = params.erosion
+    ep.max_steps, ep.pit_steps, ep.evap_rate = max_steps, 100000, evap_rate
+    g, z, rng = gpu_window(arr), np.zeros(P), np.random.default_rng(5)
+    x, y = 12.0 + rng.random(P), 12.0 + rng.random(P)
+    return lambda: gm.apply_spawns(g, ep, np.zeros(P, np.int64), x, y, z, z, 1.0, wave=P)
+
+
+def test_waiting_droplets_do_not_hold_up_the_hand_offs(cuda):
+    # four times the droplets on the one cell: four times the hand-offs one after another, and no dearer ones
+    few, many = (_kernel_us(_crowded(P, 12), "ordered_apply_kernel") for P in (2048, 8192))
+    assert many / few < 5.0, (few, many)
