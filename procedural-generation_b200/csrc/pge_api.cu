@@ -374,6 +374,7 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
             ow.vals_in = ws_ptr<int32_t>(ws, lay.w_vals0);
             ow.vals_out = ws_ptr<int32_t>(ws, lay.w_vals1);
             for (int k = 0; k < 3; k++) ow.fin[k] = ws_ptr<float>(ws, lay.w_fin[k]);
+            ow.tails = ws_ptr<uint32_t>(ws, lay.w_fin[0]);
             ow.temp = ws_ptr<void>(ws, lay.w_temp);
             ow.temp_bytes = lay.w_temp_bytes;
             ow.offsets = lay.cap >= COMPACT_CAP ? ws_ptr<long long>(ws, lay.w_offsets) : nullptr;

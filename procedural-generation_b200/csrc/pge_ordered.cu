@@ -130,11 +130,12 @@ __device__ __forceinline__ void cp_wait()
 // key = the slot's cell (invalid past a list's end); the slots enter the stable sort in (droplet,
 // entry) order, so equal cells keep the serial order
 __global__ void ordered_keys_kernel(long long nslots, int cap, const int32_t *cell, const int64_t *count,
-                                    SortKey invalid, SortKey *keys, int32_t *vals, unsigned int *ticket)
+                                    SortKey invalid, SortKey *keys, int32_t *vals, uint32_t *tails, unsigned int *ticket)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nslots; s += (long long)gridDim.x * blockDim.x) {
         const long long q = s / cap, k = s - q * cap;
+        if ((s & 31) == 0) tails[s >> 5] = 0;
         keys[s] = k < count[q] ? (SortKey)cell[s] : invalid;
         vals[s] = (int32_t)s;
     }
@@ -142,11 +143,13 @@ __global__ void ordered_keys_kernel(long long nslots, int cap, const int32_t *ce
 
 // the entries of a wave's lists compacted in (droplet, entry) order: entry k of droplet q goes to offsets[q] + k
 __global__ void ordered_compact_keys_kernel(long long nslots, int cap, const int32_t *cell, const int64_t *count,
-                                            const long long *offsets, SortKey *keys, int32_t *vals, unsigned int *ticket)
+                                            const long long *offsets, SortKey *keys, int32_t *vals, uint32_t *tails,
+                                            unsigned int *ticket)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < nslots; s += (long long)gridDim.x * blockDim.x) {
         const long long q = s / cap, k = s - q * cap;
+        if ((s & 31) == 0) tails[s >> 5] = 0;
         if (k < count[q]) {
             const long long e = offsets[q] + k;
             keys[e] = (SortKey)cell[s];
@@ -166,12 +169,18 @@ __device__ __forceinline__ bool reads_next(double delta, float vol) { return vol
 
 // One warp per 32 consecutive sorted slots.  An entry's rank is the number of droplets that start between its cell's
 // first slot and it: counted in the bits of the warp's slots, after those of the slots before them where their first
-// cell's run came in from there (looked back over 128 slots at a time: only a run longer than that goes round twice).
-// (Flags, two library scans and a pass over them: 22 us a wave in six launches at N_c = 1024; as here 7.4 in one.
-// The run's first warp walking all of it: 12.4, and 68 where runs reach thousands of entries.)
+// cell's run came in from there.  The 128 slots before are counted again; beyond them, warp by warp, what each warp left
+// in `tails`: the droplets that start in its last cell's run, from the run's start (TAIL_RUN) or only in its own slots
+// (TAIL_OWN).  Nobody waits: where a warp has left nothing yet, its slots are counted again too.
+// (Flags, two library scans and a pass over them: 22 us a wave in six launches at N_c = 1024; as here 7.5 in one.
+// The run's first warp walking all of it: 12.4, and 68 where runs reach thousands of entries.  Every warp counting back
+// over the whole run, which grows with its square: 328 us for 835,000 entries on a few cells, 813 for 1.67 million, the
+// scans 35 and 57, as here 49 and 95.)
+enum : uint32_t { TAIL_OWN = 1, TAIL_RUN = 2 };
 __global__ void __launch_bounds__(256) ordered_rank_kernel(long long nslots, const SortKey *keys, const int32_t *vals, int cap,
                                                            SortKey invalid, const double *delta, const float *vol,
-                                                           const int64_t *count, const CellTerr *terr, uint32_t epoch, EntryRec *rec)
+                                                           const int64_t *count, const CellTerr *terr, uint32_t epoch,
+                                                           uint32_t *tails, EntryRec *rec)
 {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -216,14 +225,22 @@ __global__ void __launch_bounds__(256) ordered_rank_kernel(long long nslots, con
         const unsigned starts = __ballot_sync(full, k != invalid && visit(i, k));
         const SortKey k0 = __shfl_sync(full, k, 0);
         if (k0 == invalid) break;  // (the invalid slots come last)
+        const long long w0 = base >> 5;  // these slots' place in `tails`
+        const bool goes_on = __shfl_sync(full, k, 31) != invalid;
+        if (lane == 0 && goes_on) {
+            const unsigned own = cells ? starts & (full << (31 - __clz(cells))) : starts;
+            *(volatile uint32_t *)(tails + w0) = (uint32_t)__popc(own) << 2 | (cells ? TAIL_RUN : TAIL_OWN);
+        }
         uint32_t before = 0;  // droplets that start before this warp's slots at the cell whose run comes in
         if (!(cells & 1u)) {
-            bool whole = true;
-            for (long long j0 = base - 128; whole; j0 -= 128) {
+            long long w = w0;  // counted back to this warp's slots
+            auto count_128 = [&]() {
+                bool whole = true;
                 bool v[4], in[4];
+                w -= 4;
 #pragma unroll
                 for (int q = 0; q < 4; q++) {
-                    const long long j = j0 + 32 * q + lane;
+                    const long long j = 32 * (w + q) + lane;
                     in[q] = j >= 0 && keys[j] == k0;
                     v[q] = in[q] && visit(j, k0);
                 }
@@ -232,7 +249,24 @@ __global__ void __launch_bounds__(256) ordered_rank_kernel(long long nslots, con
                     before += (uint32_t)__popc(__ballot_sync(full, v[q]));
                     whole = __all_sync(full, in[q]) && whole;
                 }
+                return whole;
+            };
+            bool whole = count_128();
+            while (whole) {
+                // the 32 warps before, the nearest first; one whose last slot is of another cell ends the run
+                const long long t = w - 1 - lane;
+                const bool in = t >= 0 && keys[32 * t + 31] == k0;
+                const uint32_t tail = in ? *(volatile uint32_t *)(tails + t) : (uint32_t)TAIL_RUN;
+                const unsigned run = __ballot_sync(full, (tail & 3u) == TAIL_RUN), none = __ballot_sync(full, (tail & 3u) == 0);
+                const int to_run = run ? __ffs(run) - 1 : 32, to_none = none ? __ffs(none) - 1 : 32;
+                const bool ends = to_run < to_none;
+                before += __reduce_add_sync(full, lane < to_none && lane <= to_run ? tail >> 2 : 0u);
+                if (ends) break;
+                w -= to_none;
+                if (to_none == 0) whole = count_128();
             }
+            if (lane == 0 && goes_on && !cells)
+                *(volatile uint32_t *)(tails + w0) = (before + (uint32_t)__popc(starts)) << 2 | TAIL_RUN;
         }
         if (k == invalid) continue;
         const unsigned upto = full >> (31 - lane);
@@ -879,17 +913,17 @@ cudaError_t ordered_wave(const OrderedWave &w, cudaStream_t st)
         if ((e = cudaMemcpyAsync(&total, w.offsets + w.nw, sizeof(long long), cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
         ordered_compact_keys_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.cap, w.a.cell, w.a.count, w.offsets, w.keys_in,
-                                                                      w.vals_in, w.a.ticket);
+                                                                      w.vals_in, w.tails, w.a.ticket);
         nslots = total;
     } else {
         ordered_keys_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.cap, w.a.cell, w.a.count, w.invalid, w.keys_in, w.vals_in,
-                                                              w.a.ticket);
+                                                              w.tails, w.a.ticket);
     }
     tb = w.temp_bytes;
     e = cub::DeviceRadixSort::SortPairs(w.temp, tb, w.keys_in, w.keys_out, w.vals_in, w.vals_out, (int)nslots, 0, w.end_bit, st);
     if (e != cudaSuccess) return e;
     ordered_rank_kernel<<<grid_for(nslots), 256, 0, st>>>(nslots, w.keys_out, w.vals_out, w.cap, w.invalid, w.a.delta, w.a.vol, w.a.count,
-                                                          w.a.terr, w.a.epoch, const_cast<EntryRec *>(w.a.rec));
+                                                          w.a.terr, w.a.epoch, w.tails, const_cast<EntryRec *>(w.a.rec));
     const bool lake = w.a.lakes && w.a.R;
     const int blocks = (int)w.nw;  // a warp per droplet
     if (w.a.ecap && lake)

@@ -114,6 +114,7 @@ struct OrderedWave {
     SortKey *keys_in, *keys_out;
     int32_t *vals_in, *vals_out;
     float *fin[3];  // the finish's gathered rows, a float a slot each
+    uint32_t *tails;  // the ranks' count of each 32 sorted slots' last run (the finish's rows are free until the finish)
     void *temp;
     size_t temp_bytes;
     // long lists: the recorded entries compacted before the ranks (nullptr: every slot goes through them);

@@ -42,3 +42,10 @@ def test_waiting_droplets_do_not_hold_up_the_hand_offs(cuda):
     # four times the droplets on the one cell: four times the hand-offs one after another, and no dearer ones
     few, many = (_kernel_us(_crowded(P, 12), "ordered_apply_kernel") for P in (2048, 8192))
     assert many / few < 5.0, (few, many)
+
+
+def test_ranks_grow_with_the_entries(cuda):
+    # eight times the entries on the same few cells: eight times the slots to rank (sixty-four, if every slot went over
+    # the whole of its cell's run)
+    short, long_ = (_kernel_us(_crowded(2048, steps, 1e-4), "ordered_rank_kernel") for steps in (100, 800))
+    assert long_ / short < 8.0, (short, long_)
