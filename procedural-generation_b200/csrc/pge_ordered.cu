@@ -328,76 +328,114 @@ __global__ void park_keys_kernel(long long nitems, int cap, const int32_t *cell,
     }
 }
 
-// The warp that holds a lake's first item walks the lake's parks in the serial order: the lake takes what it still has
-// room for, the rest is refused.  The reads of 32 parks at a time are in flight together and only the room is counted
-// down one after another; parks on one cell add to its load in their order (no other lake touches the cell).
+// A warp takes 32 sorted items and the lakes whose first park is among them; a lake takes what it still has room for,
+// the rest is refused, and the room is counted down in the serial order.  The warp reads its items together; the lakes
+// whose parks all lie within them are walked in shared memory by the lane of their first, all at once.  A lake with parks
+// beyond them (at most the last) is walked by the whole warp, 32 parks at a time, their reads in flight together and only
+// the room counted down one after another.  Parks on one cell add to its load in their order (no other lake touches the
+// cell).
 //
-// Bound by the longest lake's parks.  A thread walking its lake's, every read behind the one before: 34 to 292 us a wave
-// on five N_c = 256 worlds; as here at most 41.
+// Bound by the reads' latency and the longest lake's parks.  A wave of 2048 droplets, all the parks in lakes of one cell /
+// of 37 / of 500 / in one lake, us: a thread walking its lake's, every read behind the one before 5.0 / 16 / 95 / 1460;
+// the whole warp for each lake in turn 44 / 15 / 12 / 137; as here 5.3 / 5.9 / 12 / 132.
 constexpr int PARK_THREADS = 64, PARK_WARPS = PARK_THREADS / 32;
+struct ParkItems {
+    double sent[32], taken[32], rest[32];
+};
 __global__ void __launch_bounds__(PARK_THREADS) park_walk_kernel(long long nitems, int cap, const uint32_t *keys, const int32_t *vals,
                                                                  const int32_t *cell, const double *delta, const int32_t *park_k,
                                                                  double *lake_room, double *lake_load, double *rest)
 {
-    __shared__ double sent[PARK_WARPS][32], taken[PARK_WARPS][32];
+    __shared__ ParkItems items[PARK_WARPS];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    double *sd = sent[threadIdx.x >> 5], *tk = taken[threadIdx.x >> 5];
+    ParkItems &w = items[threadIdx.x >> 5];
     const long long nwarps = (long long)gridDim.x * PARK_WARPS;
+    // the item at sorted place t (a park with a lake: its entry index was checked by park_keys_kernel): its load to
+    // shared memory
+    auto load_item = [&](long long t, int32_t &v, int32_t &c) {
+        v = vals[t];
+        const long long s = (long long)(v / LAKE_PARKS) * cap + park_k[v];
+        c = cell[s];
+        w.sent[lane] = delta[s];
+    };
+    // what the item at this lane was refused, and what its cell takes: the lanes of a cell, all in `mine`, in their order
+    auto settle = [&](unsigned mine, int32_t v, int32_t c) {
+        rest[v] = w.rest[lane];
+        unsigned same = __match_any_sync(mine, c);
+        if (lane == __ffs(same) - 1) {
+            double load = lake_load[c];
+            for (; same; same &= same - 1) {
+                const double take = w.taken[__ffs(same) - 1];
+                if (take > 0.0) load += take;
+            }
+            lake_load[c] = load;
+        }
+    };
+    // one item counted down from its lake's room: what the lake takes of it
+    auto count_down = [&](double &room, double sent, double &refused) {
+        double take = sent;
+        refused = 0.0;
+        if (take > room) {
+            refused = take - room;
+            take = room;
+        }
+        if (take > 0.0) room -= take;
+        return take;
+    };
     for (long long base = ((long long)blockIdx.x * PARK_WARPS + (threadIdx.x >> 5)) * 32; base < nitems; base += nwarps * 32) {
         const long long i = base + lane;
         const uint32_t key = i < nitems ? keys[i] : 0xffffffffu;
-        unsigned heads = __ballot_sync(full, key != 0xffffffffu && (i == 0 || keys[i - 1] != key));
-        while (heads) {
-            const int hl = __ffs(heads) - 1;
-            heads &= heads - 1;
-            const uint32_t lake = __shfl_sync(full, key, hl);
-            double room = lake_room[lake];
-            for (long long t0 = base + hl;; t0 += 32) {
-                const long long t = t0 + lane;
-                const bool in = t < nitems && keys[t] == lake;
-                const unsigned mine = __ballot_sync(full, in);  // a prefix of the lanes (keys are sorted)
-                const int n = __popc(mine);
-                int32_t v = 0, c = 0;
-                if (in) {
-                    v = vals[t];  // a park with a lake (its entry index checked by park_keys_kernel)
-                    const long long s = (long long)(v / LAKE_PARKS) * cap + park_k[v];
-                    c = cell[s];
-                    sd[lane] = delta[s];
-                }
-                __syncwarp();
-                double my_take = 0.0, my_rest = 0.0;
-                for (int k = 0; k < n; k++) {
-                    double take = sd[k], r = 0.0;
-                    if (take > room) {
-                        r = take - room;
-                        take = room;
-                    }
-                    if (take > 0.0) room -= take;
-                    if (k == lane) {
-                        my_take = take;
-                        my_rest = r;
-                    }
-                }
-                tk[lane] = my_take;
-                __syncwarp();
-                if (in) {
-                    rest[v] = my_rest;
-                    unsigned same = __match_any_sync(mine, c);
-                    if (lane == __ffs(same) - 1) {
-                        double load = lake_load[c];
-                        for (; same; same &= same - 1) {
-                            const double take = tk[__ffs(same) - 1];
-                            if (take > 0.0) load += take;
-                        }
-                        lake_load[c] = load;
-                    }
-                }
-                __syncwarp();
-                if (n < 32) break;
-            }
-            if (lane == 0) lake_room[lake] = room;
+        const bool head = key != 0xffffffffu && (i == 0 || keys[i - 1] != key);
+        const unsigned heads = __ballot_sync(full, head), valid = __ballot_sync(full, key != 0xffffffffu);
+        if (!heads) continue;
+        // the last lake goes on beyond these items (no lake sorts last, so they are then all valid)
+        const uint32_t key31 = __shfl_sync(full, key, 31);
+        const bool open = valid == full && base + 32 < nitems && keys[base + 32] == key31;
+        const int first = __ffs(heads) - 1, last = 31 - __clz(heads), end = open ? last : __popc(valid);
+        // ---- the lakes within the items
+        const bool in = lane >= first && lane < end;
+        const unsigned mine = __ballot_sync(full, in);
+        int32_t v = 0, c = 0;
+        if (in) load_item(i, v, c);
+        __syncwarp();
+        if (in && head) {
+            const unsigned later = lane < 31 ? heads >> (lane + 1) : 0u;
+            const int to = later ? lane + __ffs(later) : end;
+            double room = lake_room[key];
+            for (int k = lane; k < to; k++) w.taken[k] = count_down(room, w.sent[k], w.rest[k]);
+            lake_room[key] = room;
         }
+        __syncwarp();
+        if (in) settle(mine, v, c);
+        __syncwarp();
+        if (!open) continue;
+        // ---- the lake that goes on
+        double room = lake_room[key31];
+        for (long long t0 = base + last;; t0 += 32) {
+            const long long t = t0 + lane;
+            const bool at = t < nitems && keys[t] == key31;
+            const unsigned theirs = __ballot_sync(full, at);  // a prefix of the lanes (keys are sorted)
+            const int n = __popc(theirs);
+            if (at) load_item(t, v, c);
+            __syncwarp();
+            double my_take = 0.0, my_rest = 0.0;
+            for (int k = 0; k < n; k++) {
+                double refused;
+                const double take = count_down(room, w.sent[k], refused);
+                if (k == lane) {
+                    my_take = take;
+                    my_rest = refused;
+                }
+            }
+            w.taken[lane] = my_take;
+            w.rest[lane] = my_rest;
+            __syncwarp();
+            if (at) settle(theirs, v, c);
+            __syncwarp();
+            if (n < 32) break;
+        }
+        if (lane == 0) lake_room[key31] = room;
     }
 }
 

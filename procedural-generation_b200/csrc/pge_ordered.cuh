@@ -91,7 +91,6 @@ struct ParkWave {
     double *rest;                    // out: per park the rest refused
     uint32_t *keys_in, *keys_out;
     int32_t *vals_in, *vals_out;
-    int end_bit;
     void *temp;
     size_t temp_bytes;
 };

@@ -49,3 +49,20 @@ def test_ranks_grow_with_the_entries(cuda):
     # the whole of its cell's run)
     short, long_ = (_kernel_us(_crowded(2048, steps, 1e-4), "ordered_rank_kernel") for steps in (100, 800))
     assert long_ / short < 8.0, (short, long_)
+
+
+def test_lakes_of_one_park_are_walked_together(cuda):
+    # a few dozen parks: as many lakes of one park each cost about what one lake of them all does (one after another
+    # they took more than four times as long)
+    from tests.test_gpu_many_lakes import lake_blocks, spawns
+
+    def walk(cells_a_lake):
+        g, ep = lake_blocks(96, cells_a_lake)
+        g.lake_room.fill_(1e9)
+        sp = spawns(40, 96)
+        us = _kernel_us(lambda: gm.apply_spawns(g, ep, *sp, 1.0, wave=40, parks=True), "park_walk_kernel")
+        assert int((g.lake_load > 0).sum()) > 20
+        return us
+
+    each, one = walk(1), walk(0)
+    assert each / one < 2.5, (each, one)
