@@ -58,7 +58,6 @@ inline int grid_for(long long n, int threads = 256)
 }
 
 constexpr int kSpinLimit = 1 << 24;  // ~ seconds of looks and sleeps: far beyond any real hand-off
-constexpr int POLL_EVERY = 256;      // looks between two at whether another wait has given up (a power of two)
 
 // A cell's hand-off word: 16 bytes, two 8-byte halves (acc low 32 bits | count << 32) and (acc high
 // 32 bits | count << 32), where acc is the live net change and count the hand-off counter.  Each
@@ -467,6 +466,7 @@ constexpr int REC_RING = 128;
 // droplets: at most 16 of them 3290 / 9406 / 22,843 / 103,940 (the looks then hold up the hand-offs), 256 of them
 // 3040 / 5710 / 11,110 / 43,510; waves spread over the terrain are the same with either (2048 droplets: 832, 825).
 constexpr uint32_t BACK_NS = 64, BACK_MAX = 256;
+constexpr int LONGEST = 4 + (int)BACK_MAX / 8;  // what four looks and the longest sleep count
 
 template <int N>
 struct Int {
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(32) ordered_apply_kernel(const OrderedArgs a)
         ulonglong2 wc;
         const bool late = !ok;
         if (late) {
-            for (int i = 0, waited = 0; !ok; i++) {
+            for (int i = 0; !ok; i++) {  // (i: the looks, and the sleeps at eight BACK_NS a look)
                 if (need_a && !hand_ready(wa.x, wa.y, A.turn)) hand_load(a.hand + A.cell, wa.x, wa.y);
                 hand_load(a.hand + B.cell, wb.x, wb.y);
                 hand_load(a.hand + C.cell, wc.x, wc.y);
@@ -701,11 +701,10 @@ __global__ void __launch_bounds__(32) ordered_apply_kernel(const OrderedArgs a)
                     if (away > 1) {
                         const uint32_t n = away < BACK_MAX ? away - 1 : BACK_MAX;
                         __nanosleep(n * BACK_NS);
-                        waited += (int)(n >> 3);  // (a look takes about eight of them)
+                        i += (int)(n >> 3 & ~3u);
                     }
-                    waited += 4;
-                    if (waited >= kSpinLimit || ((i & (POLL_EVERY - 1)) == POLL_EVERY - 1 && *(volatile int *)a.error)) {
-                        if (waited >= kSpinLimit) atomicExch(a.error, 1);
+                    if (i >= kSpinLimit || ((i & 255) >= 256 - LONGEST && *(volatile int *)a.error)) {
+                        if (i >= kSpinLimit) atomicExch(a.error, 1);
                         return false;  // this wait, or another one, gave up
                     }
                 }
