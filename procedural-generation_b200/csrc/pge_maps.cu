@@ -340,14 +340,20 @@ struct ThermalArgs {
 // One pass, a tile a block: the tile's surface and three cells around it in shared memory, then in turn every cell's
 // flows to its neighbours and their scale (two cells around), the share of its inflow a submerged cell has room for
 // (one cell around), and the cells' new height and sediment -- the reference's three sweeps (particle.py:1107-1227) in
-// its order of additions.  A flow and the one back share a distance, so a cell keeps four; the metric is the six faces'
-// alike, so a block takes its tile of every face in turn where the grid still fills the GPU (TH_FILL blocks).
+// its order of additions.  A flow and the one back share a distance, so a cell keeps four.
 //
-// Bound by shared-memory reads and float64 arithmetic, not by memory.  N_c = 1024, talus and creep: 1069 us as three
+// Bound by shared-memory reads and float64 arithmetic, not by memory.  N_c = 1024, talus and creep: 1050 us as three
 // sweeps of HBM and a copy (every neighbour's mask, surface and metric read and its distance's root taken 24 times a
-// cell); as tiles 464 with each flow computed again wherever it is used, 462 with the flows in shared memory, 406 with
-// a thread's own flows in registers and its neighbours' already at their scale.
-constexpr int TH_I = 16, TH_J = 32, TH_THREADS = TH_I * TH_J, TH_FILL = 592;
+// cell); as tiles of 16 x 32 464 with each flow computed again wherever it is used, 462 with the flows in shared memory,
+// 427 with a thread's own flows in registers and its neighbours' already at their scale; tiles of 16 x 16 400, of
+// 8 x 32 or 8 x 16 417.  The tile stays below the 48 KB a block may have without a function attribute: setting one
+// waits until no other thread of the process is in a launch, and a thread that runs a pass of many waves is in one
+// nearly all the time (64 worlds together, six iterations each: 3.0 to 4.2 s with the attribute set a call, 2.25).
+//
+// The metric is the six faces' alike, so a block takes its tile of every face in turn where one face's tiles fill the
+// GPU (TH_FILL: four blocks on each of 148 multiprocessors), us, a face a block / in turn: N_c = 256 (289 tiles a face)
+// 58 / 64, 320 (441) 75 / 71, 512 (1089) 144 / 127, 1024 (4225) 500 / 400.
+constexpr int TH_I = 16, TH_J = 16, TH_THREADS = TH_I * TH_J, TH_FILL = 592;
 constexpr int TH_RING = (TH_I + 4) * (TH_J + 4) - TH_THREADS;  // the two cells around the tile
 struct ThermalTile {
     double sent[8][TH_I + 4][TH_J + 4];  // a cell's flow to each neighbour at its scale
@@ -359,10 +365,9 @@ struct ThermalTile {
 
 // MASKED: some cells may be frozen or outside (a mask, or the creep pass's submerged cells)
 template <bool MASKED>
-__global__ void __launch_bounds__(TH_THREADS, 2) thermal_tile_kernel(const ThermalArgs t, int faces)
+__global__ void __launch_bounds__(TH_THREADS, 4) thermal_tile_kernel(const ThermalArgs t, int faces)
 {
-    extern __shared__ __align__(16) unsigned char th_smem[];
-    ThermalTile &T = *reinterpret_cast<ThermalTile *>(th_smem);
+    __shared__ ThermalTile T;
     const int NE = t.NE, i0 = blockIdx.y * TH_I, j0 = blockIdx.x * TH_J;
     constexpr int DI[8] = {1, 1, 0, -1, -1, -1, 0, 1}, DJ[8] = {0, 1, 1, 1, 0, -1, -1, -1};  // k + 4 is opposite k
     const double half_rate = 0.5 * t.rate;
@@ -496,14 +501,6 @@ __global__ void __launch_bounds__(TH_THREADS, 2) thermal_tile_kernel(const Therm
     }
 }
 
-template <bool MASKED>
-void thermal_launch(const ThermalArgs &t, dim3 grid, int faces, cudaStream_t st)
-{
-    const int smem = (int)sizeof(ThermalTile);
-    cudaFuncSetAttribute(thermal_tile_kernel<MASKED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    thermal_tile_kernel<MASKED><<<grid, TH_THREADS, smem, st>>>(t, faces);
-}
-
 __global__ void copy2_kernel(long long n, const double *a, const double *b, double *da, double *db)
 {
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
@@ -540,9 +537,9 @@ void thermal_on_scratch(const PgeGrid &g, PgeState &s, double *tb, long long n, 
         grid.z = 1;
     }
     if (t.mask)
-        thermal_launch<true>(t, grid, faces, st);
+        thermal_tile_kernel<true><<<grid, TH_THREADS, 0, st>>>(t, faces);
     else
-        thermal_launch<false>(t, grid, faces, st);
+        thermal_tile_kernel<false><<<grid, TH_THREADS, 0, st>>>(t, faces);
     if (!(creep_rate > 0.0)) {
         copy2_kernel<<<grid_for(n), 256, 0, st>>>(n, tb, tb + n, s.height, s.sediment);
         return;
@@ -554,7 +551,7 @@ void thermal_on_scratch(const PgeGrid &g, PgeState &s, double *tb, long long n, 
     t.rate = creep_rate;
     t.new_h = s.height;
     t.new_s = s.sediment;
-    thermal_launch<true>(t, grid, faces, st);
+    thermal_tile_kernel<true><<<grid, TH_THREADS, 0, st>>>(t, faces);
 }
 
 void thermal(const PgeGrid &g, PgeState &s, const Layout &lay, void *ws, double rate, double creep_rate, double cap, float soft,
