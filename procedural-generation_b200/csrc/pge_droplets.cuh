@@ -622,6 +622,9 @@ __device__ __forceinline__ void sync_own(LCell &x, const LCell &changed)
 // 1.6 million droplets (N_c = 1024): 22.5 ms with deaths and refills as they come; finals an entry an iteration 20.6,
 // and none applied once there is nothing to place 20.1; refills of 2, 4 and 8 lanes 18.9, 18.0, 17.8; lists closed
 // with them, for 4, 6 and 10 lanes, 17.1, 16.8, 16.8.
+// What it costs is a step's latency where few droplets live long (2048 of 510 steps each: 2.80 ms, 2.91 with the finals
+// ahead of the step's code and the list's end told apart in every entry's arithmetic, 2.87 as here; one droplet a step
+// 3.3 us, 3.6 and 3.5).
 // ---------------------------------------------------------------------------
 constexpr int REFILL_LANES = 6;
 enum { ST_DROP, ST_STEPS, ST_ENTRIES, ST_CLAMPED, ST_OVER, ST_TOPEND, ST_DEFICIT, ST_LOSTOFF, ST_ERODED, ST_DEPOSITED,
@@ -799,26 +802,7 @@ __global__ void __launch_bounds__(256, MINB) droplet_kernel(const DropArgs a)
         bool moved = false;
         bool last = false;  // the list is at its end
         Entry en;
-        if (LEDGER && fin >= 0) {
-            if (fin >= 2 && !TAPE && !a.rec_cell && L.surplus == 0.0) {
-                // nothing left to place: the deposits still to come, the pending one among them, change nothing
-                rec_n += nout - fin;
-                has_pe = false;
-                last = true;
-            } else if (fin < nout) {
-                load_lcell(a, t, r0, cur);
-                en.cell = r0;
-                en.delta = fin == 0 ? load : 0.0;
-                en.vol = -1.0f;
-                en.ma = en.mb = 0.0f;
-                en.sidx = -1;
-                have_entry = true;
-                r0 = r1; r1 = r2; r2 = r3; r3 = r4; r4 = r5; r5 = r6; r6 = r7;
-                fin++;
-            } else {
-                last = true;
-            }
-        } else do {
+        if (!LEDGER || fin < 0) do {
             if (step >= p.max_steps) { cause = PGE_DEATH_AGE; break; }
             const int m = cv.m;
             if (m == PGE_MASK_OUTSIDE) { exited = true; cause = PGE_DEATH_EXIT; break; }
@@ -1131,11 +1115,35 @@ __global__ void __launch_bounds__(256, MINB) droplet_kernel(const DropArgs a)
                 uphill = 0;
             }
         } while (false);
+        else {
+            if (fin >= 2 && !TAPE && !a.rec_cell && L.surplus == 0.0) {
+                // nothing left to place: the deposits still to come, the pending one among them, change nothing
+                rec_n += nout - fin;
+                has_pe = false;
+                last = true;
+            } else if (fin < nout) {
+                load_lcell(a, t, r0, cur);
+                en.cell = r0;
+                en.delta = fin == 0 ? load : 0.0;
+                en.vol = -1.0f;
+                en.ma = en.mb = 0.0f;
+                en.sidx = -1;
+                have_entry = true;
+                r0 = r1; r1 = r2; r2 = r3; r3 = r4; r4 = r5; r5 = r6; r6 = r7;
+                fin++;
+            } else {
+                last = true;
+                // no next cell: one that limits nothing (a floor below, a ceiling above every surface)
+                cur.cell = -1;
+                cur.hs = pe.delta < 0.0 ? -__longlong_as_double(0x7ff0000000000000ll) : __longlong_as_double(0x7ff0000000000000ll);
+                cur.accws = cur.own = 0.0;
+            }
+        }
 
         // ---- the ledger, one entry behind the trace
         if (LEDGER && has_pe && (have_entry || last)) {
             // `cur` still describes the cell the entry was made at
-            apply_entry<TAPE, ROUTE>(a, t, L, pe, pend, !last, cur, trow);
+            apply_entry<TAPE, ROUTE>(a, t, L, pe, pend, true, cur, trow);
             sync_own(cur, pend);
             sync_own(nxt, pend);
         }
