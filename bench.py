@@ -455,7 +455,10 @@ def run_b200(args, rank, world_size, dist):
         batched = run_batched(args, rank, world_size, dist, dev)
     if rank != 0:
         return None
-    # the routing surface of the evolved N_c = 1024 terrain (erosion.flood_every's refresh), CUDA-event timed
+    # the routing surface of the evolved N_c = 1024 terrain (erosion.flood_every's refresh), CUDA-event timed; a first
+    # call makes the owner table and loads the kernels
+    st.refresh_route(float(params.erosion.route_eps) / st.height_unit_m)
+    torch.cuda.synchronize()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record()
     sweeps = st.refresh_route(float(params.erosion.route_eps) / st.height_unit_m)
@@ -651,7 +654,7 @@ def main():
     ap.add_argument("--alt-steps", type=int, default=5)
     ap.add_argument("--no-brush", action="store_true", help="skip the brush (radius 3) measurement")
     ap.add_argument("--no-f32", action="store_true", help="skip the float32-trace measurement")
-    ap.add_argument("--apply-lanes", type=int, default=0, help="ordered apply: droplets per warp (0 = 1)")
+    ap.add_argument("--apply-lanes", type=int, default=0, help="accepted and without effect: the ordered apply runs one droplet per warp")
     ap.add_argument("--config", default="c2", choices=("c2", "c5"),
                     help="c2: the Earth-default N_c=1024 line (default); c5: the N_c=8192 planet level on one GPU")
     ap.add_argument("--planet-iterations", type=int, default=0, help="c5: run this many iterations as the timed stage")

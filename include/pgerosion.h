@@ -437,8 +437,8 @@ PGE_API int pge_route_flood(const PgeGrid *g, const PgeState *s, const int32_t *
  * component, -1 above the waterline).  Components are joined along the
  * owner relation taken both ways (the reference walks it one way from each
  * component's lowest cell; they differ only where a cube corner's halo
- * mapping is one-sided).  One pass: *sweeps (host, may be NULL) gets 1;
- * spherical grids only. */
+ * mapping is one-sided).  One pass: max_sweeps (>= 1) is accepted and
+ * without effect, *sweeps (host, may be NULL) gets 1; spherical grids only. */
 PGE_API int pge_sea_base(const PgeGrid *g, const PgeState *s, const int32_t *owner, const float *area, double min_area, double *base,
                          int32_t *labels, int64_t max_sweeps, int64_t *sweeps, void *ws, size_t ws_bytes, void *stream);
 

@@ -383,14 +383,13 @@ int run_waves(const PgeGrid *g, PgeState *s, const PgeSpawns *sp, const PgeParam
                                          : s->route ? droplet_blocks_per_sm_f64_route(32, false)
                                          : p->precision == PGE_PREC_F64 ? droplet_blocks_per_sm_f64(32, 1, false)
                                                                       : droplet_blocks_per_sm_f32(32, 1, false));
-            // a float64 wave whose droplets fit the GPU as one warp each (2368) takes the trace of one warp a droplet:
-            // waves of 2048: 184 against 305 us (N_c = 1024), 297 against 493 with lakes, 316 against 505 with
-            // banks; of 4096: 315 against 303, 369 against 544, 329 against 539; of 8192: 523 against 352, 486 against
-            // 646 (some 6000 with lakes).  A thread's step with a route or banks is that much longer, so there the
-            // line lies at twice the residents.
+            // A float64 wave of up to twice as many droplets as the GPU holds at once as one warp each (2368) takes the
+            // trace of one warp a droplet; larger ones a thread a droplet.  us a wave of 2368 / 4000 / 4736 / 6000 / 8192
+            // droplets, a warp and a thread: N_c = 128 sphere 189 249 278 315 358 and 242 329 343 384 430; N_c = 512
+            // 190 300 331 382 469 and 285 320 329 354 363; with lakes (N_c = 256) 333 401 430 460 545 and 560 638 679 701
+            // 754; a window with banks 307 435 450 553 675 and 474 546 505 575 605.
             const long long warp_waves = p->precision == PGE_PREC_F64 && p->trace_lanes == 0
-                                             ? (long long)sm_count() * trace_blocks_per_sm_f64(s->route != nullptr, lateral) *
-                                                   (s->route || lateral ? 2 : 1)
+                                             ? 2ll * sm_count() * trace_blocks_per_sm_f64(s->route != nullptr, lateral)
                                              : 0;
             int ebits = 1;
             while ((1LL << ebits) <= wave) ebits++;

@@ -452,7 +452,7 @@ __device__ __forceinline__ void load_lcell(const DropArgs &a, const Table &t, lo
 }
 
 // Apply one change-list entry (particle.py:934-1018) at cell `c` against the
-// droplet's view of the terrain.  `nx` is the next entry's cell (has_next).
+// droplet's view of the terrain.  `nx` is the next entry's cell (at the list's end one that limits nothing).
 // Updates c.own (and the table), emits the atomics and returns the applied
 // change (0 when nothing moved).
 template <bool TAPE>
@@ -467,7 +467,7 @@ __device__ __forceinline__ void tape_entry(const DropArgs &a, Ledger &L, long lo
 }
 
 template <bool TAPE = false, bool ROUTE = false>
-__device__ __forceinline__ void apply_entry(const DropArgs &a, Table &t, Ledger &L, const Entry &e, LCell &c, bool has_next,
+__device__ __forceinline__ void apply_entry(const DropArgs &a, Table &t, Ledger &L, const Entry &e, LCell &c,
                                             const LCell &nx, long long row = 0)
 {
     const PgeParams &p = a.p;
@@ -502,12 +502,10 @@ __device__ __forceinline__ void apply_entry(const DropArgs &a, Table &t, Ledger 
             const float2 rc = __ldg(a.R + c.cell);
             if (rc.y >= 1.5f && (double)rc.x > floor_) floor_ = (double)rc.x;
         }
-        if (has_next) {
-            const double ns = nx.live();
-            if (ns > floor_) {
-                floor_ = ns;
-                fsrc = 4;
-            }
+        const double ns = nx.live();
+        if (ns > floor_) {
+            floor_ = ns;
+            fsrc = 4;
         }
         if (e_act > s_c - floor_) {
             e_act = s_c - floor_;
@@ -547,7 +545,7 @@ __device__ __forceinline__ void apply_entry(const DropArgs &a, Table &t, Ledger 
             has_ref = L.has_prev;
             ref_live = L.prev_live;
             ref_cell = L.prev_cell;
-        } else if (has_next) {
+        } else {
             has_ref = true;
             ref_live = nx.live();
             ref_cell = nx.cell;
@@ -1143,7 +1141,7 @@ __global__ void __launch_bounds__(256, MINB) droplet_kernel(const DropArgs a)
         // ---- the ledger, one entry behind the trace
         if (LEDGER && has_pe && (have_entry || last)) {
             // `cur` still describes the cell the entry was made at
-            apply_entry<TAPE, ROUTE>(a, t, L, pe, pend, true, cur, trow);
+            apply_entry<TAPE, ROUTE>(a, t, L, pe, pend, cur, trow);
             sync_own(cur, pend);
             sync_own(nxt, pend);
         }
@@ -1181,7 +1179,7 @@ __global__ void __launch_bounds__(256, MINB) droplet_kernel(const DropArgs a)
             bk.cell = bank_en.cell;
             if (LEDGER) {
                 load_lcell(a, t, bank_en.cell, bk);
-                apply_entry<TAPE, ROUTE>(a, t, L, pe, pend, true, bk, trow);
+                apply_entry<TAPE, ROUTE>(a, t, L, pe, pend, bk, trow);
                 sync_own(bk, pend);
                 sync_own(cur, pend);
                 sync_own(nxt, pend);

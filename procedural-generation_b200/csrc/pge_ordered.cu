@@ -59,10 +59,12 @@ inline int grid_for(long long n, int threads = 256)
 
 constexpr int kSpinLimit = 1 << 24;  // ~ seconds of looks and sleeps: far beyond any real hand-off
 
-// A cell's hand-off word: 16 bytes, two 8-byte halves (acc low 32 bits | count << 32) and (acc high
-// 32 bits | count << 32), where acc is the live net change and count the hand-off counter.  Each
-// half is one single-copy-atomic 64-bit access, so a reader that sees the same count in both halves
-// holds a consistent word, however the 16 bytes were read.
+// A cell's hand-off word: 16 bytes, two 8-byte halves (acc low 32 bits | count << 32) and (acc high 32 bits | count <<
+// 32), where acc is the live net change and count the hand-off counter.  A reader that sees the same count in both
+// halves holds one whole word as long as each half is one: PTX promises that of the relaxed loads and stores below
+// (64-bit single-copy atomicity).  The copies ahead (`send`) are asynchronous, weak reads, of which it does not say so;
+// they read 16 aligned bytes of one 32-byte sector, which this GPU moves as one.  A copy that is old, or torn between
+// the halves, fails the test of the counts and is read again with a relaxed load.
 __device__ __forceinline__ void hand_pack(double acc, uint32_t count, unsigned long long &w0, unsigned long long &w1)
 {
     const unsigned long long bits = (unsigned long long)__double_as_longlong(acc);
@@ -773,10 +775,10 @@ __global__ void __launch_bounds__(32) ordered_apply_kernel(const OrderedArgs a)
 // ---------------------------------------------------------------------------
 // after the apply: per touched cell, in the serial (droplet, entry) order, the discharge and
 // momentum tracks (particle.py:1013-1018) and the stockpile (:1019-1041); then the cell's net
-// change to the accumulators and its packed samples (:1005-1009); and the wave's eroded and
-// deposited totals (integer fixed point, so their order does not matter).  First every sorted slot
-// gathers what its entry adds into arrays in sorted order (one thread a slot, all loads in flight at
-// once); then one thread a cell sums its run of those arrays in order (contiguous reads).
+// change to the accumulators and its packed samples (:1005-1009).  First every sorted slot gathers
+// what its entry adds into arrays in sorted order (one thread a slot, all loads in flight at once);
+// then each cell's run of those arrays is summed in order, by a lane where it ends within 64 slots,
+// else by a whole warp.
 // ---------------------------------------------------------------------------
 __global__ void ordered_gather_kernel(const OrderedArgs a, long long nslots, const SortKey *keys, const int32_t *vals,
                                       SortKey invalid, FinishRows g)
