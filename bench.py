@@ -489,8 +489,8 @@ def run_b200(args, rank, world_size, dist):
     avg_ta = float(np.mean(ta_ms))
     achieved = per_launch_steps * BYTES_PER_STEP / (avg_ta * 1e-3) / 1e9
     # DRAM bytes per droplet pass, from ncu (dram__bytes_read.sum + dram__bytes_write.sum) over the waves of an
-    # exact pass of the N_c = 256 world: with the caches kept from kernel to kernel, as the live pass runs, 40 B
-    # a droplet-step (scaled by the pass's droplet-steps); with ncu's flush before every kernel, 33.7 MB a wave
+    # exact pass of the N_c = 256 world: with the caches kept from kernel to kernel, as the live pass runs, 35 B
+    # a droplet-step (scaled by the pass's droplet-steps); with ncu's flush before every kernel, 27.3 MB a wave
     # (the per-wave workspace is fixed, so that one scales with the waves)
     exact = apply == _lib.APPLY_ORDERED
     traffic = TRAFFIC_PER_STEP * per_launch_steps if exact else None
@@ -713,8 +713,8 @@ def main():
 DEFAULT_WAVE = 0
 #: DRAM bytes of the exact pass (trace, sort, ranks, apply, finish) per droplet-step, caches kept between
 #: kernels, and per wave with the caches flushed before every kernel; both from ncu captures of the N_c = 256 pass
-TRAFFIC_PER_STEP = 40.0
-TRAFFIC_PER_WAVE_COLD = 33.7e6
+TRAFFIC_PER_STEP = 35.0
+TRAFFIC_PER_WAVE_COLD = 27.3e6
 
 if __name__ == "__main__":
     main()

@@ -598,8 +598,8 @@ __device__ __forceinline__ void droplet_end(const OrderedArgs &a, const Walk &w,
 // copies of its records and the statistics of 32 entries at a time.
 //
 // A block takes the next droplet by a ticket, so the droplets it can wait for -- the earlier ones -- have all started,
-// in whatever order the GPU starts a wave's blocks and however few of them it holds at once (of one-warp blocks 32 a
-// multiprocessor): the earliest droplet that has not ended waits for nobody.
+// in whatever order the GPU starts a wave's blocks and however few of them it holds at once (20 a multiprocessor, by their
+// registers and shared memory): the earliest droplet that has not ended waits for nobody.
 //
 // Bound by the instructions of one entry on one warp (~110, 215-235 ns; 2048 droplets at work at once: 405), not
 // by memory.  What each choice measured, ns an entry without a wait: hand-off words read into registers ahead of

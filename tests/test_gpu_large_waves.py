@@ -1,6 +1,6 @@
 """The ordered apply where a wave has more droplets than the GPU holds at
-once (one-warp blocks: 32 a multiprocessor, 4736 of 148), so that most of its
-droplets start only when others have ended, against the oracle's trace and
+once (at most 32 one-warp blocks a multiprocessor, 4736 of 148), so that many
+of its droplets start only when others have ended, against the oracle's trace and
 serial apply (IEEE float64 in the same order: heights identical in 99.9 % of
 the cells, everything within 1e-5, the clamped count equal)."""
 import ctypes
