@@ -42,7 +42,7 @@ def test_map_passes_run_beside_exact_passes(cuda, run):
     threads = [threading.Thread(target=exact_pass, args=w) for w in worlds]
     for t in threads:
         t.start()
-    time.sleep(0.3)
+    time.sleep(0.15)
     t0 = time.perf_counter()
     with torch.cuda.stream(mine):
         for _ in range(3):
