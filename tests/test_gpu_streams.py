@@ -36,13 +36,20 @@ def test_map_passes_run_beside_exact_passes(cuda, run):
     for _ in range(4):
         arr, params = window_world("tilt", N=N)
         worlds.append((gpu_window(arr), params.erosion, torch.cuda.Stream()))
-    with torch.cuda.stream(mine):  # (a first call makes tables and the workspace)
+
+    def start():
+        threads = [threading.Thread(target=exact_pass, args=w) for w in worlds]
+        for t in threads:
+            t.start()
+        return threads
+
+    for t in start():  # (a first call makes tables and the workspaces)
+        t.join()
+    with torch.cuda.stream(mine):
         passes[run]()
     torch.cuda.synchronize()
-    threads = [threading.Thread(target=exact_pass, args=w) for w in worlds]
-    for t in threads:
-        t.start()
-    time.sleep(0.15)
+    threads = start()
+    time.sleep(0.2)
     t0 = time.perf_counter()
     with torch.cuda.stream(mine):
         for _ in range(3):
